@@ -9,7 +9,8 @@
 //      cooperative launch); the resident engine, for mixed PCG with one
 //      right-hand side when the system fits it;
 //      for FP64 PCG with one right-hand side, also the graph engine with the
-//      fused iteration (one cooperative kernel an iteration, k_pcg_fused);
+//      fused iteration (k_pcg_fused, k_pcg_fused_loop) and the on-chip
+//      engine;
 //   2. when the graph engine leads with three kernels an iteration: its best
 //      shape with the SpMV phases' L2 prefetch 1, 2 or 4 rounds ahead.
 // Each candidate solves the caller's right-hand side once untimed (the graph
@@ -96,7 +97,7 @@ bool file_lookup(const std::string &key, Tuned *t) {
                     "engine=%d threads=%d spw=%d pf=%d fused=%d ms=%lf", &e, &th, &sp, &pf, &fu,
                     &ms) == 6 &&
         (e == 1 || e == 2 || e == 4) && (th == 128 || th == 256) && sp >= 0 && sp <= 64 &&
-        pf >= 0 && pf <= 8 && fu >= 0 && fu <= 4) {
+        pf >= 0 && pf <= 8 && fu >= 0 && fu <= kFusedOnChip) {
       t->engine = e;
       t->threads = th;
       t->spw = sp;
@@ -192,7 +193,7 @@ extern "C" int sfr_gpu_autotune(sfr_system *s, int32_t solver, int32_t k, const 
   for (int th : {256, 128})
     for (int sp : {0, 2, 8}) add({2, th, sp, 0, 0});
   if (precision == SFR_FP64 && solver == SFR_PCG && k == 1) {
-    for (int mode : {1, 2, 3, 4}) add({2, 256, 0, 0, mode});
+    for (int mode : {1, 2, 3, 4, kFusedOnChip}) add({2, 256, 0, 0, mode});
   }
   add({1, 0, 0, 0, 0});
   if (precision == SFR_MIXED && solver == SFR_PCG && k == 1 && own_diag && resident_fits(s))

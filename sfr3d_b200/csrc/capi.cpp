@@ -436,6 +436,8 @@ int sfr_gpu_destroy(sfr_system *s) {
   cudaFree(s->d_rdelta);
   cudaFree(s->d_rbad);
   cudaFree(s->ws.base);
+  if (s->ev0) cudaEventDestroy(s->ev0);
+  if (s->ev1) cudaEventDestroy(s->ev1);
   if (s->stream) cudaStreamDestroy(s->stream);
   delete s;
   return SFR_OK;

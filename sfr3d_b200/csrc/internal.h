@@ -12,6 +12,7 @@
 namespace sfr {
 
 constexpr int kWarpHost = 32;  // rows per SELL slice (one warp)
+constexpr int kFusedOnChip = 5;  // sfr_system::graph_fused: the on-chip engine
 
 // SELL-32 layout built on the host from one of the reference's layouts.
 // src[e] is the index of slot e's value in the value source the caller
@@ -103,9 +104,12 @@ struct sfr_system {
   int32_t graph_threads = 256;   // graph engine launch shape
   int32_t graph_spw = 0;         // SELL slices per warp; 0: one wave of resident blocks
   int32_t graph_pf = 0;          // SpMV-phase L2 prefetch distance (rounds); 0: off
-  int32_t graph_fused = 4;       // FP64 PCG, one RHS: the fused iteration's mode (4: one launch a solve)
+  // FP64 PCG, one RHS: 0 three kernels an iteration, 1-4 the fused iteration's
+  // modes, kFusedOnChip the on-chip engine (mode 4 where it does not fit)
+  int32_t graph_fused = sfr::kFusedOnChip;
   int32_t graph_stage = 0;       // BiCGSTAB SpMV phases: slices staged in shared memory
   std::vector<sfr::Tuned> tuned; // autotuned choices, used when engine == 0
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // around a solve's launch (onchip.cu)
   int64_t bytes = 0;
 };
 
@@ -154,6 +158,11 @@ int wait_selftest_resident(int32_t absent, uint32_t spin_limit, cudaStream_t st)
 bool resident_fits(sfr_system *s);
 int solve_resident(sfr_system *s, const double *d_b, double *d_x, double tol, uint32_t maxit,
                    int32_t newx, cudaStream_t st, sfr_solve_info *info);
+
+// On-chip engine (onchip.cu): FP64 PCG, one right-hand side.  SFR_UNSUPPORTED
+// when the system fits neither of its forms.
+int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double *d_x, double tol,
+                 uint32_t maxit, int32_t newx, cudaStream_t st, sfr_solve_info *info);
 
 // BiCGSTAB(2), GMRES(15), MINRES (krylov_ext.cu): one right-hand side, FP64;
 // d_diag null means the system's own diagonal

@@ -866,6 +866,8 @@ int enqueue_team_fp64(sfr_system *s, int32_t solver, const double *d_b, double *
 int auto_engine(sfr_system *s, int32_t solver, int32_t k, int32_t precision, bool own_diag) {
   const bool resident_case = precision == SFR_MIXED && solver == SFR_PCG && k == 1 && own_diag;
   if (resident_case && s->n >= kGraphEngineRows && resident_fits(s)) return 4;
+  if (precision == SFR_FP64 && solver == SFR_PCG && k == 1 && s->graph_fused == kFusedOnChip)
+    return 2;  // the on-chip engine, at every size
   return s->n >= kGraphEngineRows ? 2 : 1;
 }
 
@@ -899,6 +901,12 @@ int solve_device(sfr_system *s, int32_t solver, int32_t k, const double *d_diag_
     // automatic choice: a diagonal that is not positive has no Jacobi scaling
     if (rc != SFR_UNSUPPORTED || (engine == 4 && !tuned)) return rc;
   }
+  if ((engine == 0 || engine == 2) && precision == SFR_FP64 && solver == SFR_PCG && k == 1 &&
+      fused == kFusedOnChip) {
+    const int rc = solve_onchip(s, d_diag_k, d_b, d_x, tol, maxit, newx, st, info);
+    if (rc != SFR_UNSUPPORTED) return rc;
+  }
+  if (fused == kFusedOnChip) fused = 4;
   if (engine == 0 || engine == 4) engine = s->n >= kGraphEngineRows ? 2 : 1;
   if (engine == 2 || engine == 3)
     return solve_stream(s, solver, k, d_diag_k, d_b, d_x, tol, maxit, newx, precision,
