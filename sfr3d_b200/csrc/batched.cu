@@ -36,6 +36,7 @@ struct sfr_batch {
   sfr_batch_tune tune{};        // the last autotune's report
   // launch plan
   int32_t plan_solver = -1, plan_precision = -1, grid = 0;
+  bool onchip = false;  // the plan runs on the on-chip engine
   sfr::TeamTable table{};
   int4 *d_block = nullptr;
   int2 *d_sys = nullptr;
@@ -95,9 +96,83 @@ std::vector<int> share_by_weight(const sfr_batch *b, int gmax) {
   return nb;
 }
 
+// Blocks a system's team needs at least: one, or on the on-chip engine as
+// many as hold its rows.
+std::vector<int> least_blocks(const sfr_batch *b, bool onchip) {
+  std::vector<int> nb(b->nsys, 1);
+  const int most = onchip ? team_max_slices_onchip(b->device) : 0;
+  if (onchip && most > 0)
+    for (int s = 0; s < b->nsys; ++s) nb[s] = std::max(1, (b->nslices[s] + most - 1) / most);
+  return nb;
+}
+
+// FP64 PCG runs on the on-chip engine's teams when every system has room
+// there; the persistent kernels take the rest (and more systems).
+bool onchip_fits(const sfr_batch *b, int32_t solver, int32_t precision) {
+  if (solver != SFR_PCG || precision != SFR_FP64) return false;
+  const int gmax = team_max_grid_onchip(b->device);
+  if (gmax <= 0 || team_max_slices_onchip(b->device) <= 0) return false;
+  int64_t total = 0;
+  for (int v : least_blocks(b, true)) total += v;
+  return total <= gmax;
+}
+
 int max_grid(const sfr_batch *b, int32_t solver, int32_t precision) {
+  if (onchip_fits(b, solver, precision)) return team_max_grid_onchip(b->device);
   return precision == SFR_MIXED ? team_max_grid_mixed(solver, b->device)
                                 : team_max_grid_fp64(solver, b->device);
+}
+
+// Blocks per team on the on-chip engine: the shares that minimise the
+// slowest team's predicted time
+//   t(B) = iterations (f + w slices / B),   f = 3.2 us (1.2 us for one block)
+//                                           w = 0.1 us
+// where weight = slices x iterations.  f is the exchange and the publication
+// of p, which more blocks do not shrink; w a slice's share of an iteration
+// with two blocks an SM (88^3 on one system: 7.4 us for 144 slices an SM).
+// 24 boxes of 8 to 48 cells, host buffers: 4.86 ms, against 11.7 ms on the
+// persistent kernels' teams.
+std::vector<int> share_by_model(const sfr_batch *b, int gmax) {
+  const int S = b->nsys;
+  const std::vector<int> least = least_blocks(b, true);
+  auto time = [&](int s, int B) {
+    const double it = b->weight[s] / b->nslices[s];
+    return it * ((B > 1 ? 3.2 : 1.2) + 0.1 * b->nslices[s] / B);
+  };
+  auto need = [&](int s, double T) {  // the fewest blocks within T
+    const int most = b->nslices[s];
+    int B = least[s];
+    if (time(s, B) <= T) return B;
+    const double it = b->weight[s] / b->nslices[s], rest = T / it - 3.2;
+    if (rest <= 0.0) return INT32_MAX;
+    B = std::max(std::max(least[s], 2), static_cast<int>(std::ceil(0.1 * most / rest - 1e-9)));
+    return B > most ? INT32_MAX : B;
+  };
+  auto fits = [&](double T) {
+    int64_t total = 0;
+    for (int s = 0; s < S && total <= gmax; ++s) total += need(s, T);
+    return total <= gmax;
+  };
+  double hi = 0.0, lo = 0.0;
+  for (int s = 0; s < S; ++s) hi = std::max(hi, time(s, least[s]));
+  for (int i = 0; i < 60; ++i) {
+    const double mid = 0.5 * (lo + hi);
+    (fits(mid) ? hi : lo) = mid;
+  }
+  std::vector<int> nb(S);
+  int total = 0;
+  for (int s = 0; s < S; ++s) total += nb[s] = need(s, hi);
+  while (total < gmax) {  // leftovers to the teams predicted slowest
+    int worst = -1;
+    for (int s = 0; s < S; ++s)
+      if (nb[s] < b->nslices[s] && time(s, nb[s] + 1) < time(s, nb[s]) &&
+          (worst < 0 || time(s, nb[s]) > time(worst, nb[worst])))
+        worst = s;
+    if (worst < 0) break;
+    ++nb[worst];
+    ++total;
+  }
+  return nb;
 }
 
 // Install a launch plan: team s gets nb[s] blocks (b->team_blocks when set
@@ -110,17 +185,20 @@ int plan(sfr_batch *b, int32_t solver, int32_t precision) {
     return SFR_UNSUPPORTED;
   }
   const int S = b->nsys;
+  b->onchip = onchip_fits(b, solver, precision);
+  auto share = [&] { return b->onchip ? share_by_model(b, gmax) : share_by_weight(b, gmax); };
   std::vector<int> nb;
   int total = 0;
   if (static_cast<int>(b->team_blocks.size()) == S) {
     nb = b->team_blocks;
+    const std::vector<int> least = least_blocks(b, b->onchip);
     for (int s = 0; s < S; ++s) {
-      nb[s] = std::max(1, std::min(nb[s], b->nslices[s]));
+      nb[s] = std::max(least[s], std::min(nb[s], b->nslices[s]));
       total += nb[s];
     }
-    if (total > gmax) nb = share_by_weight(b, gmax);
+    if (total > gmax) nb = share();
   } else {
-    nb = share_by_weight(b, gmax);
+    nb = share();
   }
   total = 0;
   for (int v : nb) total += v;
@@ -150,8 +228,9 @@ int plan(sfr_batch *b, int32_t solver, int32_t precision) {
           cudaSuccess ||
       cudaMemcpy(b->d_sys, sys.data(), sizeof(int2) * grid, cudaMemcpyHostToDevice) != cudaSuccess)
     return SFR_CUDA_ERROR;
-  const size_t need = precision == SFR_MIXED ? team_ws_bytes_mixed(b->cat.n, grid)
-                                             : team_ws_bytes_fp64(b->cat.n, grid);
+  const size_t need = b->onchip                ? team_ws_bytes_onchip(b->cat.n, grid)
+                      : precision == SFR_MIXED ? team_ws_bytes_mixed(b->cat.n, grid)
+                                               : team_ws_bytes_fp64(b->cat.n, grid);
   if (need > b->ws_bytes) {
     cudaFree(b->ws);
     b->ws = nullptr;
@@ -185,7 +264,9 @@ int capture(sfr_batch *b, int32_t solver, int32_t precision, double tol, uint32_
   if (cudaMemsetAsync(b->d_bar, 0, sizeof(unsigned) * 2 * b->nsys, cs) != cudaSuccess)
     rc = SFR_CUDA_ERROR;
   if (rc == SFR_OK)
-    rc = precision == SFR_MIXED
+    rc = b->onchip ? enqueue_team_onchip(&b->cat, b->d_b, b->d_x, tol, maxit, newx, b->table,
+                                         b->grid, b->ws, b->d_out, b->d_ctl, cs)
+         : precision == SFR_MIXED
              ? enqueue_team_mixed(&b->cat, solver, b->d_b, b->d_x, tol, maxit, newx, b->table,
                                   b->grid, b->ws, b->d_out, b->d_ctl, cs)
              : enqueue_team_fp64(&b->cat, solver, b->d_b, b->d_x, tol, maxit, newx, b->table,
@@ -284,6 +365,8 @@ int sfr_gpu_batch_create(int32_t nsys, const int32_t *neq, const int32_t *nad,
       cat.col.push_back(h.col[e] + static_cast<int32_t>(rows));
       cat.src.push_back(h.src[e] >= 0 ? h.src[e] + static_cast<int32_t>(src) : -1);
     }
+    cat.bandwidth = std::max(cat.bandwidth, h.bandwidth);
+    cat.max_width = std::max(cat.max_width, h.max_width);
     rows += static_cast<int64_t>(h.nslices) * sfr::kWarpHost;
     slices += h.nslices;
     src += ns;

@@ -67,6 +67,20 @@ struct ChipArgs {
   int newx;
 };
 
+// The blocks that solve one system together, and this block's part: slices
+// [s0, s1) of the system's [first, first + count), which the team's blocks
+// [b0, b1) share in order.  A launch for one system is one team.
+struct ChipTeam {
+  int s0, s1, first, count, b0, b1;
+  int row_end;  // the system's rows end here
+  int sys;
+  unsigned long long t0;  // the block's start (global_ns)
+  __device__ __forceinline__ int owner(int row) const {
+    const long long B = b1 - b0, ns = count, sl = row / kWarp - first;
+    return b0 + static_cast<int>(((sl + 1) * B + ns - 1) / ns - 1);
+  }
+};
+
 // Four values summed over a warp with six 64-bit shuffles (a butterfly that
 // halves the values a lane carries before it halves the lanes): lane l ends
 // with the total of value l >> 3, the same bits in all eight of its lanes.
@@ -144,7 +158,7 @@ struct Scalars {
 
 // The result record of a finished solve.
 __device__ __forceinline__ void put_result(SolveOut *out, const Scalars &sc,
-                                           const double (&tot)[4]) {
+                                           const double (&tot)[4], double ms) {
   SolveOut o{};
   o.iters = static_cast<int>(sc.iters);
   o.status = sc.status;
@@ -154,6 +168,7 @@ __device__ __forceinline__ void put_result(SolveOut *out, const Scalars &sc,
   o.norm_r = sqrt(tot[3]);
   o.conv = sc.conv;
   o.inner_iters = static_cast<int>(sc.iters);
+  o.team_ms = ms;
   *out = o;
 }
 
@@ -177,8 +192,8 @@ __device__ __forceinline__ bool ld_slot(const ulonglong2 *p, double *v, unsigned
   return hi == epoch;
 }
 
-// Totals of four values over the grid, in every thread, the same bits in all
-// blocks.  Each block writes its totals with the epoch beside each value;
+// Totals of four values over the team, in every thread, the same bits in all
+// its blocks.  Each block writes its totals with the epoch beside each value;
 // thread b of every block polls block b's slot, so the values arrive with
 // the poll: one L2 round trip.  Two buffers alternate: a block writes epoch e
 // only after it read every block's epoch e - 1, which each published after it
@@ -187,17 +202,25 @@ __device__ __forceinline__ bool ld_slot(const ulonglong2 *p, double *v, unsigned
 // block records SFR_TIMEOUT in *err, and a block that sees *err set stops
 // waiting.  False on either.  sm: 32 * 4 + 4 doubles, bad: a shared word.
 template <bool kFence>
-__device__ __forceinline__ bool grid_sum4(const ChipArgs &a, unsigned &epoch,
+__device__ __forceinline__ bool grid_sum4(const ChipArgs &a, const ChipTeam &t, unsigned &epoch,
                                           const double (&acc)[4], double (&tot)[4], double *sm,
                                           int *bad) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int G = gridDim.x;
+  const int G = t.b1 - t.b0;
   ++epoch;
-  ChipSlot *cur = a.slots + static_cast<size_t>(epoch & 1u) * G;
   const double s = block_sum4(acc, sm);
+  if (G == 1) {  // a team of one block: no other block to tell
+    if (warp == 0 && (lane & 7) == 0) sm[(lane >> 3) * 32] = s;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) tot[i] = sm[i * 32];
+    __syncthreads();
+    return true;
+  }
+  ChipSlot *cur = a.slots + static_cast<size_t>(epoch & 1u) * gridDim.x + t.b0;
   if (warp == 0 && (lane & 7) == 0) {
     if (kFence) cuda::atomic_thread_fence(cuda::memory_order_release, cuda::thread_scope_device);
-    st_slot(&cur[blockIdx.x].v[lane >> 3], s, epoch);
+    st_slot(&cur[blockIdx.x - t.b0].v[lane >> 3], s, epoch);
   }
   if (threadIdx.x == 0) *bad = 0;
   __syncthreads();  // sm is free again; *bad is 0
@@ -228,31 +251,32 @@ __device__ __forceinline__ bool grid_sum4(const ChipArgs &a, unsigned &epoch,
     }
     __syncwarp();
     if (kFence) cuda::atomic_thread_fence(cuda::memory_order_acquire, cuda::thread_scope_device);
-    const double t = warp_sum4(v);
-    if ((lane & 7) == 0) sm[(lane >> 3) * 32 + warp] = t;
+    const double q = warp_sum4(v);
+    if ((lane & 7) == 0) sm[(lane >> 3) * 32 + warp] = q;
   }
   __syncthreads();
   const int ww = watchers >> 5;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    double t = sm[i * 32];
-    for (int w = 1; w < ww; ++w) t += sm[i * 32 + w];
-    tot[i] = t;
+    double q = sm[i * 32];
+    for (int w = 1; w < ww; ++w) q += sm[i * 32 + w];
+    tot[i] = q;
   }
   const bool ok = *bad == 0;
   __syncthreads();
   return ok;
 }
 
-// The blocks [lo, hi] owning the columns this block's rows gather from.
+// The blocks [range[0], range[1]] owning the columns this block gathers from.
 template <typename I>
-__device__ __forceinline__ void gather_range(const int *sm_sp, const I *cols, int s0, int s1,
-                                             int nslices, int *range) {
+__device__ __forceinline__ void gather_range(const ChipTeam &t, const int *sm_sp, const I *cols,
+                                             int *range) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  int cmin = s0 * kWarp, cmax = s1 * kWarp - 1;
-  for (int s = s0 + warp; s < s1; s += nw) {
+  int cmin = t.s0 * kWarp, cmax = t.s1 * kWarp - 1;
+  for (int s = t.s0 + warp; s < t.s1; s += nw) {
     const int row = s * kWarp + lane;
-    for (int e = sm_sp[s - s0] + lane; e < sm_sp[s - s0 + 1]; e += kWarp) {
+    if (row >= t.row_end) continue;  // padding: its columns mean nothing
+    for (int e = sm_sp[s - t.s0] + lane; e < sm_sp[s - t.s0 + 1]; e += kWarp) {
       const int c = slot_col(cols, e, row);
       cmin = min(cmin, c);
       cmax = max(cmax, c);
@@ -266,9 +290,7 @@ __device__ __forceinline__ void gather_range(const int *sm_sp, const I *cols, in
   atomicMin(range, cmin);
   atomicMax(range + 1, cmax);
   __syncthreads();
-  const int lo = min(owner_block(range[0], nslices), static_cast<int>(blockIdx.x));
-  const int hi = max(owner_block(min(range[1], nslices * kWarp - 1), nslices),
-                     static_cast<int>(blockIdx.x));
+  const int lo = t.owner(range[0]), hi = t.owner(range[1]);
   __syncthreads();
   if (threadIdx.x == 0) {
     range[0] = lo;
@@ -287,7 +309,9 @@ __device__ __forceinline__ void gather_range(const int *sm_sp, const I *cols, in
 //   kKeep    in L2, under its normal policy
 //   kStream  from HBM, evict-first
 constexpr int kLevels = 4;
-constexpr int kLevelBytes[kLevels] = {8, 16, 24, 40};
+__host__ __device__ constexpr int level_bytes(int level) {
+  return level == 0 ? 8 : level == 1 ? 16 : level == 2 ? 24 : 40;
+}
 enum Slots { kHold, kKeep, kStream };
 
 // Threads a block: 24 warps at 80 registers hold a slice's slots, gathers and
@@ -296,22 +320,27 @@ enum Slots { kHold, kKeep, kStream };
 // 17.3 / 51.5.
 constexpr int kGridThreads = 768;
 
+// A block's static shared memory.
+struct GridShared {
+  double red[32 * 4];
+  int bad, range[2];
+};
+
 template <typename I, int kLevel, Slots kSlots>
-__global__ void __launch_bounds__(kGridThreads, 1) pcg_grid_kernel(const ChipArgs a) {
-  extern __shared__ double sm_dyn[];
-  __shared__ double red[32 * 4];
-  __shared__ int bad, range[2];
+__device__ __forceinline__ void pcg_grid_body(const ChipArgs &a, const ChipTeam &t,
+                                              double *sm_dyn, GridShared &sh) {
+  double *const red = sh.red;
+  int *const bad = &sh.bad, *const range = sh.range;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  int s0, s1;
-  block_slices(a.nslices, &s0, &s1);
+  const int s0 = t.s0, s1 = t.s1;
   const int r0 = s0 * kWarp, rows = (s1 - s0) * kWarp;
-  const int own = max(0, min(rows, a.n - r0));  // rows that are equations
+  const int own = max(0, min(rows, t.row_end - r0));  // rows that are equations
   const int slot0 = __ldg(a.sptr + s0);
   double *sm_t = sm_dyn;
   double *vz = kLevel >= 1 ? sm_t + rows : a.z + r0;
   double *vx = kLevel >= 2 ? sm_t + 2 * rows : a.x + r0;
   double *sm_d = sm_t + 3 * rows, *sm_p = sm_d + rows;  // level 3
-  double *sm_v = sm_t + (kLevelBytes[kLevel] / 8) * rows;  // kHold
+  double *sm_v = sm_t + (level_bytes(kLevel) / 8) * rows;  // kHold
   const I *cols = cols_of<I>(SlotCols{a.col, a.off});
   const int held = kSlots == kHold ? __ldg(a.sptr + s1) - slot0 : 0;  // a multiple of 32
   I *sm_c = reinterpret_cast<I *>(sm_v + held);
@@ -322,7 +351,8 @@ __global__ void __launch_bounds__(kGridThreads, 1) pcg_grid_kernel(const ChipArg
     sm_c[i] = ld_stream(cols + slot0 + i);
   }
   __syncthreads();
-  gather_range(sm_sp, cols, s0, s1, a.nslices, range);
+  const bool alone = t.b1 - t.b0 == 1;
+  if (!alone) gather_range(t, sm_sp, cols, range);
 
   unsigned epoch = 0, tick = 0;
   double acc[4], tot[4];
@@ -333,7 +363,7 @@ __global__ void __launch_bounds__(kGridThreads, 1) pcg_grid_kernel(const ChipArg
     for (int s = s0 + warp; s < s1; s += nw) {
       const int base = sm_sp[s - s0], w = (sm_sp[s - s0 + 1] - base) >> 5;
       const int row = s * kWarp + lane, lr = row - r0;
-      if (row >= a.n) continue;
+      if (row >= t.row_end) continue;
       const double pr = kLevel == 3 ? sm_p[lr] : ld_vec(a.p + row);
       const double dg = kLevel == 3 ? sm_d[lr] : __ldcg(a.diag + row);
       const double zr = vz[lr];
@@ -385,6 +415,10 @@ __global__ void __launch_bounds__(kGridThreads, 1) pcg_grid_kernel(const ChipArg
   // p is complete: wait on the blocks whose p this block gathers (a block has
   // at least as many threads as the grid has blocks, so every range fits)
   auto publish = [&]() {
+    if (alone) {
+      __syncthreads();
+      return true;
+    }
     return neighbour_wait(a.ticks, a.err, a.spin_limit, ++tick, range[0], range[1]);
   };
 
@@ -400,13 +434,13 @@ __global__ void __launch_bounds__(kGridThreads, 1) pcg_grid_kernel(const ChipArg
     vz[lr] = z;
     put_p(lr, a.newx ? z : x0);
   }
-  if (!grid_sum4<true>(a, epoch, acc, tot, red, &bad)) return;
+  if (!grid_sum4<true>(a, t, epoch, acc, tot, red, bad)) return;
   Scalars sc(a.tol * sqrt(fabs(tot[0])));
   if (!a.newx) {
     matvec([&](int lr, double y, double, double d, double) {
       vz[lr] = xdiv(xsub(ld_vec(a.b + r0 + lr), y), d);
     });
-    if (!grid_sum4<false>(a, epoch, acc, tot, red, &bad)) return;  // every gather of x0 is done
+    if (!grid_sum4<false>(a, t, epoch, acc, tot, red, bad)) return;  // every gather of x0 is done
     for (int lr = threadIdx.x; lr < own; lr += blockDim.x) put_p(lr, vz[lr]);
     if (!publish()) return;
   }
@@ -414,14 +448,14 @@ __global__ void __launch_bounds__(kGridThreads, 1) pcg_grid_kernel(const ChipArg
   for (unsigned j = 0;; ++j) {
     acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
     matvec([&](int lr, double y, double p, double d, double z) {
-      const double t = xdiv(y, d);
-      sm_t[lr] = t;
+      const double mq = xdiv(y, d);
+      sm_t[lr] = mq;
       acc[0] += y * p;
       acc[1] += y * z;
-      acc[2] += y * t;
+      acc[2] += y * mq;
       acc[3] += (d * z) * z;
     });
-    if (!grid_sum4<false>(a, epoch, acc, tot, red, &bad)) return;
+    if (!grid_sum4<false>(a, t, epoch, acc, tot, red, bad)) return;
     if (!sc.next(tot, j, a.maxit)) break;
     const double alpha = sc.alpha, beta = sc.beta;
     for (int lr = threadIdx.x; lr < own; lr += blockDim.x) {
@@ -449,8 +483,57 @@ __global__ void __launch_bounds__(kGridThreads, 1) pcg_grid_kernel(const ChipArg
     acc[2] += r * xdiv(r, d);
     acc[3] += r * r;
   });
-  if (!grid_sum4<false>(a, epoch, acc, tot, red, &bad)) return;
-  if (blockIdx.x == 0 && threadIdx.x == 0) put_result(a.out, sc, tot);
+  if (!grid_sum4<false>(a, t, epoch, acc, tot, red, bad)) return;
+  if (static_cast<int>(blockIdx.x) == t.b0 && threadIdx.x == 0)
+    put_result(a.out + t.sys, sc, tot, (global_ns() - t.t0) * 1e-6);
+}
+
+// One system over the whole grid.
+template <typename I, int kLevel, Slots kSlots>
+__global__ void __launch_bounds__(kGridThreads, 1) pcg_grid_kernel(const ChipArgs a) {
+  extern __shared__ double sm_dyn[];
+  __shared__ GridShared sh;
+  ChipTeam t{};
+  block_slices(a.nslices, &t.s0, &t.s1);
+  t.count = a.nslices;
+  t.b1 = gridDim.x;
+  t.row_end = a.n;
+  t.t0 = global_ns();
+  pcg_grid_body<I, kLevel, kSlots>(a, t, sm_dyn, sh);
+}
+
+// Many systems, a team of blocks each (batched.cu's table).  A block picks
+// its level by its own rows: blocks of one team need not agree, they only
+// exchange sums and p.  Two blocks an SM: twice the teams, and a small
+// system's share is a finer one.
+constexpr int kTeamThreads = 384;
+
+template <typename I>
+__global__ void __launch_bounds__(kTeamThreads, 2) pcg_team_kernel(const ChipArgs a,
+                                                                   const TeamTable tt, int smem) {
+  extern __shared__ double sm_dyn[];
+  __shared__ GridShared sh;
+  const int4 e = tt.block[blockIdx.x];
+  const int2 y = tt.sys[blockIdx.x];
+  ChipTeam t;
+  t.s0 = e.x;
+  t.s1 = e.y;
+  t.b0 = e.z;
+  t.b1 = e.w;
+  t.first = tt.block[e.z].x;
+  t.count = tt.block[e.w - 1].y - t.first;
+  t.sys = y.x;
+  t.row_end = y.y;
+  t.t0 = global_ns();
+  const int slices = t.s1 - t.s0, rows = slices * kWarp;
+  const int left = smem - 4 * (slices + 1);
+  const int slots = a.sptr[t.s1] - a.sptr[t.s0];
+  if (rows * level_bytes(3) + slots * static_cast<int>(8 + sizeof(I)) <= left)
+    pcg_grid_body<I, 3, kHold>(a, t, sm_dyn, sh);
+  else if (rows * level_bytes(2) <= left)
+    pcg_grid_body<I, 2, kKeep>(a, t, sm_dyn, sh);
+  else
+    pcg_grid_body<I, 0, kKeep>(a, t, sm_dyn, sh);
 }
 
 // ---- cluster form --------------------------------------------------------
@@ -632,7 +715,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) pcg_cluster_kernel(const C
     acc[3] += r * r;
   });
   cluster_sum4(ex, buf, acc, tot, red);
-  if (blockIdx.x == 0 && threadIdx.x == 0) put_result(a.out, sc, tot);
+  if (blockIdx.x == 0 && threadIdx.x == 0) put_result(a.out, sc, tot, 0.0);
 }
 
 // ---- host ------------------------------------------------------------------
@@ -784,7 +867,7 @@ bool grid_shape(const sfr_system *s, Shape *sh) {
   const int slices = (ns + g - 1) / g, rows = slices * kWarp;
   const int threads = std::max((g + kWarp - 1) / kWarp * kWarp, std::min(kGridThreads, rows));
   auto fixed = [&](int level) {
-    return static_cast<size_t>(rows) * kLevelBytes[level] + sizeof(int) * (slices + 1);
+    return static_cast<size_t>(rows) * level_bytes(level) + sizeof(int) * (slices + 1);
   };
   const size_t hold = fixed(3) + static_cast<size_t>(rows) * s->A.max_width * (8 + sizeof(I));
   if (hold <= limit) {
@@ -809,7 +892,89 @@ bool grid_shape(const sfr_system *s, Shape *sh) {
   return true;
 }
 
+// Dynamic shared memory of a team block: two to an SM.
+size_t team_smem(int device) {
+  int per_sm = 0;
+  if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) !=
+      cudaSuccess)
+    return 0;
+  // a block also takes its static shared memory and the system's 1 KB
+  const int half = per_sm / 2 - 1024 - static_cast<int>(kGridStatic);
+  return half > 0 ? static_cast<size_t>(half) / 256 * 256 : 0;
+}
+
+size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
+
 }  // namespace
+
+int team_max_slices_onchip(int device) {
+  const size_t b = team_smem(device);
+  return b ? static_cast<int>((b - 8) / (kWarp * level_bytes(0) + 4)) : 0;
+}
+
+int team_max_grid_onchip(int device) {
+  const size_t b = team_smem(device);
+  int occ = INT32_MAX;
+  for (const void *k : {reinterpret_cast<const void *>(pcg_team_kernel<int16_t>),
+                        reinterpret_cast<const void *>(pcg_team_kernel<int>)}) {
+    int o = 0;
+    if (!b ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(b)) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k, kTeamThreads, b) != cudaSuccess)
+      return 0;
+    occ = std::min(occ, o);
+  }
+  // neighbour_wait watches one block a thread
+  return std::min(kTeamThreads, occ * num_sms(device));
+}
+
+size_t team_ws_bytes_onchip(int n, int grid) {
+  return 2 * align256(sizeof(double) * static_cast<size_t>(n)) +
+         align256(sizeof(ChipSlot) * 2 * static_cast<size_t>(grid)) +
+         align256(64 * static_cast<size_t>(grid));
+}
+
+int enqueue_team_onchip(sfr_system *s, const double *d_b, double *d_x, double tol, uint32_t maxit,
+                        int32_t newx, const TeamTable &team, int grid, void *ws, SolveOut *d_out,
+                        unsigned *ctl, cudaStream_t st) {
+  const size_t vec = align256(sizeof(double) * static_cast<size_t>(s->n));
+  const size_t slot_b = align256(sizeof(ChipSlot) * 2 * static_cast<size_t>(grid));
+  const size_t tick_b = align256(64 * static_cast<size_t>(grid));
+  char *base = static_cast<char *>(ws);
+  ChipArgs a{};
+  a.n = s->n;
+  a.nslices = s->A.nslices;
+  a.sptr = s->A.sptr;
+  a.col = s->A.col;
+  a.off = s->A.off;
+  a.val = s->A.val;
+  a.diag = s->d_diag;
+  a.b = d_b;
+  a.x = d_x;
+  a.slots = reinterpret_cast<ChipSlot *>(base);
+  a.ticks = reinterpret_cast<unsigned *>(base + slot_b);
+  a.p = reinterpret_cast<double *>(base + slot_b + tick_b);
+  a.z = reinterpret_cast<double *>(base + slot_b + tick_b + vec);
+  a.err = reinterpret_cast<int *>(ctl + 2);
+  a.spin_limit = 1u << 22;
+  a.out = d_out;
+  a.tol = tol;
+  a.maxit = maxit;
+  a.newx = newx;
+  if (cudaMemsetAsync(base, 0, slot_b + tick_b, st) != cudaSuccess ||
+      cudaMemsetAsync(ctl, 0, 64, st) != cudaSuccess)
+    return SFR_CUDA_ERROR;
+  int smem = static_cast<int>(team_smem(s->device));
+  TeamTable tt = team;
+  void *params[] = {&a, &tt, &smem};
+  const void *k = s->A.off ? reinterpret_cast<const void *>(pcg_team_kernel<int16_t>)
+                           : reinterpret_cast<const void *>(pcg_team_kernel<int>);
+  return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kTeamThreads), params,
+                                     static_cast<size_t>(smem), st) == cudaSuccess
+             ? SFR_OK
+             : SFR_CUDA_ERROR;
+}
 
 int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double *d_x, double tol,
                  uint32_t maxit, int32_t newx, cudaStream_t st, sfr_solve_info *info) {

@@ -165,3 +165,62 @@ def test_one_step_convergence(cuda):
     assert info.status == sv.OK and info.iters <= 2
     assert rel(x, b / ad) < 1e-14
     g.close()
+
+
+def batch_of(boxes, **kw):
+    ss = [S.build(S.params(n=b, jitter=0.2, log10k=(-1.0, 1.0), seed=20 + i, **kw))
+          for i, b in enumerate(boxes)]
+    g = sv.GpuBatch([(s.neq, s.ia, s.ja) for s in ss], sv.CSRD, True)
+    g.set_values([s.al for s in ss], [s.ad for s in ss])
+    return ss, g
+
+
+# teams of one block; of one and of many; nearly as many systems as blocks;
+# rows that fill a block's shared memory in part (level 2) and past it (0)
+@pytest.mark.parametrize("boxes", [
+    [(1, 1, 1), (5, 1, 1), (33, 1, 1), (7, 6, 5)],
+    [(2, 2, 2), (40, 36, 44), (9, 9, 9), (21, 20, 19)],
+    [(4, 4, 4)] * 290,
+    [(58, 60, 62)] * 3,
+    [(97, 100, 101)] * 2], ids=["tiny", "uneven", "many", "level2", "level0"])
+def test_team_launches(cuda, boxes):
+    ss, g = batch_of(boxes)
+    xs, infos = g.solve(sv.PCG, [s.b[0] for s in ss], tol=TOL)
+    for i, (s, x, info) in enumerate(zip(ss, xs, infos)):
+        if i >= 8:
+            break
+        one = system(s)
+        want, ref = one.solve(sv.PCG, s.b[0], tol=TOL)
+        one.close()
+        assert info.status == sv.OK and abs(info.iters - ref.iters) <= 1, (i, info.iters)
+        assert rel(x, want) < BAR, i
+    assert all(i.status == sv.OK for i in infos)
+    again, _ = g.solve(sv.PCG, [s.b[0] for s in ss], tol=TOL)
+    assert all(bits_equal(a, b) for a, b in zip(xs, again))
+    # a warm start under a cap: each team's own status, as the persistent
+    # kernel gives it for that system alone (a one-row system's start is
+    # exact, and 0 / 0 a breakdown)
+    x0s = [0.999 * x for x in xs]
+    x0s[0] = xs[0]
+    xs2, infos2 = g.solve(sv.PCG, [s.b[0] for s in ss], x0s=x0s, newx=False, tol=1e-6, maxit=4,
+                          raise_on_error=False)
+    for i, (s, x, info) in enumerate(list(zip(ss, xs2, infos2))[:8]):
+        one = system(s)
+        one.set_engine(sv.ENGINE_PERSISTENT)
+        want, ref = one.solve(sv.PCG, s.b[0], x0=x0s[i], newx=False, tol=1e-6, maxit=4,
+                              raise_on_error=False)
+        one.close()
+        assert (info.status, info.iters) == (ref.status, ref.iters), i
+        assert rel(x, want) < BAR, i
+    g.close()
+
+
+def test_team_launch_with_wide_columns(cuda):
+    """A box without RCM in the batch: 32-bit columns for every system."""
+    ss, g = batch_of([(40, 40, 40), (6, 7, 8)], permute=True, rcm=False)
+    xs, infos = g.solve(sv.PCG, [s.b[0] for s in ss], tol=TOL)
+    for s, x, info in zip(ss, xs, infos):
+        ref = O.pcg(O.CSRD, True, s.ia, s.ja, s.al, s.ad, s.b[0], tol=TOL)
+        assert info.status == sv.OK and abs(info.iters - ref.iters) <= 1
+        assert rel(x, ref.x) < BAR
+    g.close()
