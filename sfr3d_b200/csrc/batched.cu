@@ -16,11 +16,13 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
 #include "internal.h"
 #include "persist.cuh"
+#include "team_plan.h"
 
 struct sfr_batch {
   int32_t device = 0;
@@ -36,10 +38,13 @@ struct sfr_batch {
   sfr_batch_tune tune{};        // the last autotune's report
   // launch plan
   int32_t plan_solver = -1, plan_precision = -1, grid = 0;
-  bool onchip = false;  // the plan runs on the on-chip engine
+  int engine = 0;  // of the plan (Engine below)
+  sfr::TeamShape shape;  // on chip: how its kernel is launched
+  float round_us = 0.f, round_us_later = 0.f;  // on chip: the rounds' times
   sfr::TeamTable table{};
   int4 *d_block = nullptr;
   int2 *d_sys = nullptr;
+  int4 *d_systems = nullptr;  // per system {first slice, slices, end row, estimated iterations}
   unsigned *d_bar = nullptr;
   void *ws = nullptr;
   size_t ws_bytes = 0;
@@ -96,62 +101,81 @@ std::vector<int> share_by_weight(const sfr_batch *b, int gmax) {
   return nb;
 }
 
-// Blocks a system's team needs at least: one, or on the on-chip engine as
-// many as hold its rows.
-std::vector<int> least_blocks(const sfr_batch *b, bool onchip) {
+// What runs a batch: the on-chip teams (PCG: onchip.cu in FP64, mixed_team.cu
+// in mixed precision) where every system has room there, else the persistent
+// kernels.
+enum Engine { kPersistent, kChipFp64, kChipMixed };
+
+// Blocks a system's team needs at least: as many as hold its rows.
+std::vector<int> least_blocks(const sfr_batch *b, const TeamShape &sh) {
   std::vector<int> nb(b->nsys, 1);
-  const int most = onchip ? team_max_slices_onchip(b->device) : 0;
-  if (onchip && most > 0)
-    for (int s = 0; s < b->nsys; ++s) nb[s] = std::max(1, (b->nslices[s] + most - 1) / most);
+  if (sh.most > 0)
+    for (int s = 0; s < b->nsys; ++s) nb[s] = std::max(1, (b->nslices[s] + sh.most - 1) / sh.most);
   return nb;
 }
 
-// FP64 PCG runs on the on-chip engine's teams when every system has room
-// there; the persistent kernels take the rest (and more systems).
-bool onchip_fits(const sfr_batch *b, int32_t solver, int32_t precision) {
-  if (solver != SFR_PCG || precision != SFR_FP64) return false;
-  const int gmax = team_max_grid_onchip(b->device);
-  if (gmax <= 0 || team_max_slices_onchip(b->device) <= 0) return false;
-  int64_t total = 0;
-  for (int v : least_blocks(b, true)) total += v;
-  return total <= gmax;
+// One block an SM while the systems are at most half as many (96^3 alone:
+// 14.6 us an iteration against 17.5 with two blocks an SM; 64 mixed boxes of
+// 8 to 96 cells 66 ms against 67), else two: twice the teams, finer shares.
+Engine pick_engine(const sfr_batch *b, int32_t solver, int32_t precision, TeamShape *shape) {
+  *shape = TeamShape{};
+  if (solver != SFR_PCG) return kPersistent;
+  const Engine e = precision == SFR_MIXED ? kChipMixed : kChipFp64;
+  for (int per_sm : {1, 2}) {
+    const TeamShape sh = e == kChipMixed ? team_shape_mixed(&b->cat, per_sm)
+                                         : team_shape_onchip(&b->cat, per_sm);
+    if (per_sm == 1 && 2 * b->nsys > num_sms(b->device)) continue;
+    int64_t total = 0;
+    for (int v : least_blocks(b, sh)) total += v;
+    if (sh.blocks > 0 && b->nsys <= kMaxTeams && total <= sh.blocks) {
+      *shape = sh;
+      return e;
+    }
+  }
+  return kPersistent;
 }
 
 int max_grid(const sfr_batch *b, int32_t solver, int32_t precision) {
-  if (onchip_fits(b, solver, precision)) return team_max_grid_onchip(b->device);
+  TeamShape sh;
+  if (pick_engine(b, solver, precision, &sh) != kPersistent) return sh.blocks;
   return precision == SFR_MIXED ? team_max_grid_mixed(solver, b->device)
                                 : team_max_grid_fp64(solver, b->device);
 }
 
-// Blocks per team on the on-chip engine: the shares that minimise the
-// slowest team's predicted time
-//   t(B) = iterations (f + w slices / B),   f = 3.2 us (1.2 us for one block)
-//                                           w = 0.1 us
-// where weight = slices x iterations.  f is the exchange and the publication
-// of p, which more blocks do not shrink; w a slice's share of an iteration
-// with two blocks an SM (88^3 on one system: 7.4 us for 144 slices an SM).
-// 24 boxes of 8 to 48 cells, host buffers: 4.86 ms, against 11.7 ms on the
-// persistent kernels' teams.
-std::vector<int> share_by_model(const sfr_batch *b, int gmax) {
+// Iterations a system is expected to take: its weight a slice, scaled so that
+// the largest estimate is the default's for that system (weights are relative).
+std::vector<double> estimates(const sfr_batch *b) {
+  std::vector<double> it(b->nsys);
+  int big = 0;
+  for (int s = 0; s < b->nsys; ++s) {
+    it[s] = b->weight[s] / b->nslices[s];
+    if (it[s] > it[big]) big = s;
+  }
+  const double scale = 15.0 * std::cbrt(static_cast<double>(b->n[big])) / it[big];
+  for (double &v : it) v = std::max(1.0, v * scale);
+  return it;
+}
+
+// Blocks per team of an on-chip launch's first round: the shares that
+// minimise the slowest team's predicted time, as next_teams does on the
+// device for the later rounds.
+std::vector<int> share_by_model(const sfr_batch *b, const TeamShape &sh) {
   const int S = b->nsys;
-  const std::vector<int> least = least_blocks(b, true);
-  auto time = [&](int s, int B) {
-    const double it = b->weight[s] / b->nslices[s];
-    return it * ((B > 1 ? 3.2 : 1.2) + 0.1 * b->nslices[s] / B);
-  };
+  const std::vector<int> least = least_blocks(b, sh);
+  const std::vector<double> it = estimates(b);
+  auto time = [&](int s, int B) { return it[s] * sh.model.us(b->nslices[s], B); };
   auto need = [&](int s, double T) {  // the fewest blocks within T
-    const int most = b->nslices[s];
-    int B = least[s];
-    if (time(s, B) <= T) return B;
-    const double it = b->weight[s] / b->nslices[s], rest = T / it - 3.2;
+    if (time(s, least[s]) <= T) return least[s];
+    const double rest = T / it[s] - sh.model.many;
     if (rest <= 0.0) return INT32_MAX;
-    B = std::max(std::max(least[s], 2), static_cast<int>(std::ceil(0.1 * most / rest - 1e-9)));
-    return B > most ? INT32_MAX : B;
+    const double B = std::max(std::max(least[s], 2) + 0.0,
+                              std::ceil(sh.model.slice * b->nslices[s] / rest - 1e-9));
+    return B > b->nslices[s] ? INT32_MAX : static_cast<int>(B);
   };
   auto fits = [&](double T) {
     int64_t total = 0;
-    for (int s = 0; s < S && total <= gmax; ++s) total += need(s, T);
-    return total <= gmax;
+    for (int s = 0; s < S && total <= sh.blocks; ++s) total += need(s, T);
+    return total <= sh.blocks;
   };
   double hi = 0.0, lo = 0.0;
   for (int s = 0; s < S; ++s) hi = std::max(hi, time(s, least[s]));
@@ -162,7 +186,7 @@ std::vector<int> share_by_model(const sfr_batch *b, int gmax) {
   std::vector<int> nb(S);
   int total = 0;
   for (int s = 0; s < S; ++s) total += nb[s] = need(s, hi);
-  while (total < gmax) {  // leftovers to the teams predicted slowest
+  while (total < sh.blocks) {  // leftovers to the teams predicted slowest
     int worst = -1;
     for (int s = 0; s < S; ++s)
       if (nb[s] < b->nslices[s] && time(s, nb[s] + 1) < time(s, nb[s]) &&
@@ -185,13 +209,17 @@ int plan(sfr_batch *b, int32_t solver, int32_t precision) {
     return SFR_UNSUPPORTED;
   }
   const int S = b->nsys;
-  b->onchip = onchip_fits(b, solver, precision);
-  auto share = [&] { return b->onchip ? share_by_model(b, gmax) : share_by_weight(b, gmax); };
+  TeamShape shape;
+  const Engine e = pick_engine(b, solver, precision, &shape);
+  b->engine = e;
+  auto share = [&] {
+    return e == kPersistent ? share_by_weight(b, gmax) : share_by_model(b, shape);
+  };
   std::vector<int> nb;
   int total = 0;
   if (static_cast<int>(b->team_blocks.size()) == S) {
     nb = b->team_blocks;
-    const std::vector<int> least = least_blocks(b, b->onchip);
+    const std::vector<int> least = least_blocks(b, shape);
     for (int s = 0; s < S; ++s) {
       nb[s] = std::max(least[s], std::min(nb[s], b->nslices[s]));
       total += nb[s];
@@ -218,6 +246,24 @@ int plan(sfr_batch *b, int32_t solver, int32_t precision) {
     }
   }
   const int grid = static_cast<int>(blocks.size());
+  const std::vector<double> est = estimates(b);
+  std::vector<int4> systems(S);
+  double longest = 0.0;
+  for (int s = 0; s < S; ++s) {
+    systems[s] = make_int4(b->slice_off[s], b->nslices[s], b->row_off[s] + b->n[s],
+                           static_cast<int>(std::min(est[s], 1e9)));
+    longest = std::max(longest, est[s] * shape.model.us(b->nslices[s], nb[s]));
+  }
+  // The first round's time, as a share of what the slowest team is predicted
+  // to take, then a quarter a round.  FP64, all of it: 24 small boxes 4.9 ms,
+  // half 5.7 (a re-plan costs the small teams more than it gives).  Mixed,
+  // half: 64 uneven boxes 72 ms (a quarter 66, all 88, one round 176), small
+  // batches 4.5 to 6.5 ms (all 3.5 to 5.6).
+  b->round_us = static_cast<float>((e == kChipMixed ? 0.5 : 1.0) * longest);
+  b->round_us_later = static_cast<float>(0.25 * longest);
+  if (cudaMemcpy(b->d_systems, systems.data(), sizeof(int4) * S, cudaMemcpyHostToDevice) !=
+      cudaSuccess)
+    return SFR_CUDA_ERROR;
   cudaFree(b->d_block);
   cudaFree(b->d_sys);
   b->d_block = nullptr;
@@ -228,7 +274,8 @@ int plan(sfr_batch *b, int32_t solver, int32_t precision) {
           cudaSuccess ||
       cudaMemcpy(b->d_sys, sys.data(), sizeof(int2) * grid, cudaMemcpyHostToDevice) != cudaSuccess)
     return SFR_CUDA_ERROR;
-  const size_t need = b->onchip                ? team_ws_bytes_onchip(b->cat.n, grid)
+  const size_t need = e == kChipFp64           ? team_ws_bytes_onchip(b->cat.n, grid, S)
+                      : e == kChipMixed        ? team_ws_bytes_mixed_team(b->cat.n, grid, S)
                       : precision == SFR_MIXED ? team_ws_bytes_mixed(b->cat.n, grid)
                                                : team_ws_bytes_fp64(b->cat.n, grid);
   if (need > b->ws_bytes) {
@@ -238,6 +285,7 @@ int plan(sfr_batch *b, int32_t solver, int32_t precision) {
     b->ws_bytes = need;
   }
   b->grid = grid;
+  b->shape = shape;
   b->table.block = b->d_block;
   b->table.sys = b->d_sys;
   b->table.bar = b->d_bar;
@@ -250,32 +298,45 @@ int plan(sfr_batch *b, int32_t solver, int32_t precision) {
   return SFR_OK;
 }
 
-// Capture [clear the team barriers -> one cooperative launch] as a graph.
-int capture(sfr_batch *b, int32_t solver, int32_t precision, double tol, uint32_t maxit,
-            int32_t newx) {
-  cudaStream_t cs = nullptr;
-  if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) return SFR_CUDA_ERROR;
+// The solve as a graph: [clear the team barriers -> one cooperative launch]
+// on the persistent kernels, rounds_graph on chip.
+int build(sfr_batch *b, int32_t solver, int32_t precision, double tol, uint32_t maxit,
+          int32_t newx) {
   cudaGraph_t g = nullptr;
   int rc = SFR_OK;
-  if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+  if (b->engine == kPersistent) {
+    cudaStream_t cs = nullptr;
+    if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess)
+      return SFR_CUDA_ERROR;
+    if (cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
+      cudaStreamDestroy(cs);
+      return SFR_CUDA_ERROR;
+    }
+    if (cudaMemsetAsync(b->d_bar, 0, sizeof(unsigned) * 2 * b->nsys, cs) != cudaSuccess)
+      rc = SFR_CUDA_ERROR;
+    if (rc == SFR_OK)
+      rc = precision == SFR_MIXED
+               ? enqueue_team_mixed(&b->cat, solver, b->d_b, b->d_x, tol, maxit, newx, b->table,
+                                    b->grid, b->ws, b->d_out, b->d_ctl, cs)
+               : enqueue_team_fp64(&b->cat, solver, b->d_b, b->d_x, tol, maxit, newx, b->table,
+                                   b->grid, b->ws, b->d_out, b->d_ctl, cs);
+    const cudaError_t ee = cudaStreamEndCapture(cs, &g);
+    if (rc == SFR_OK && ee != cudaSuccess) rc = SFR_CUDA_ERROR;
     cudaStreamDestroy(cs);
-    return SFR_CUDA_ERROR;
+  } else {
+    TeamPlan plan;
+    plan.shape = b->shape;
+    plan.table = b->table;
+    plan.systems = b->d_systems;
+    plan.nsys = b->nsys;
+    plan.grid = b->grid;
+    plan.us = b->round_us;
+    plan.us_later = b->round_us_later;
+    rc = (b->engine == kChipFp64 ? graph_team_onchip : graph_mixed_team)(
+        &b->cat, b->d_b, b->d_x, tol, maxit, newx, plan, b->ws, b->d_out, b->d_ctl, &g);
   }
-  if (cudaMemsetAsync(b->d_bar, 0, sizeof(unsigned) * 2 * b->nsys, cs) != cudaSuccess)
-    rc = SFR_CUDA_ERROR;
-  if (rc == SFR_OK)
-    rc = b->onchip ? enqueue_team_onchip(&b->cat, b->d_b, b->d_x, tol, maxit, newx, b->table,
-                                         b->grid, b->ws, b->d_out, b->d_ctl, cs)
-         : precision == SFR_MIXED
-             ? enqueue_team_mixed(&b->cat, solver, b->d_b, b->d_x, tol, maxit, newx, b->table,
-                                  b->grid, b->ws, b->d_out, b->d_ctl, cs)
-             : enqueue_team_fp64(&b->cat, solver, b->d_b, b->d_x, tol, maxit, newx, b->table,
-                                 b->grid, b->ws, b->d_out, b->d_ctl, cs);
-  const cudaError_t ee = cudaStreamEndCapture(cs, &g);
-  if (rc == SFR_OK && ee != cudaSuccess) rc = SFR_CUDA_ERROR;
   if (rc == SFR_OK && cudaGraphInstantiate(&b->exec, g, 0) != cudaSuccess) rc = SFR_CUDA_ERROR;
   if (g) cudaGraphDestroy(g);
-  cudaStreamDestroy(cs);
   if (rc == SFR_OK) {
     b->g_tol = tol;
     b->g_maxit = maxit;
@@ -296,7 +357,7 @@ int run(sfr_batch *b, int32_t solver, double tol, uint32_t maxit, int32_t newx,
       cudaGraphExecDestroy(b->exec);
       b->exec = nullptr;
     }
-    rc = capture(b, solver, precision, tol, maxit, newx);
+    rc = build(b, solver, precision, tol, maxit, newx);
     if (rc != SFR_OK) return rc;
   }
   cudaStream_t st = b->cat.stream;
@@ -326,6 +387,82 @@ int run(sfr_batch *b, int32_t solver, double tol, uint32_t maxit, int32_t newx,
 }
 
 }  // namespace
+
+TeamShape team_shape(int device, const void *kern, int threads, int per_sm, int slice_bytes,
+                     const TeamModel &model) {
+  TeamShape sh;
+  sh.per_sm = per_sm;
+  sh.threads = threads;
+  sh.model = model;
+  // an SM's shared memory over its blocks, each with the kernel's static
+  // shared memory and the 1 KB the system takes
+  int sm = 0, block = 0, occ = 0;
+  if (cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) !=
+          cudaSuccess ||
+      cudaDeviceGetAttribute(&block, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) !=
+          cudaSuccess)
+    return sh;
+  const int smem =
+      std::min(sm / per_sm - 1024, block) - static_cast<int>((sizeof(TeamShared) + 255) / 256 * 256);
+  if (smem <= 64 ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads,
+                                                    static_cast<size_t>(smem)) != cudaSuccess ||
+      occ < per_sm) {
+    (void)cudaGetLastError();  // the refusal is not a later call's error
+    return sh;
+  }
+  sh.smem = static_cast<size_t>(smem);
+  sh.most = (smem - 32) / slice_bytes;
+  // neighbour_wait watches one block a thread
+  sh.blocks = std::min(threads, per_sm * num_sms(device));
+  return sh;
+}
+
+int rounds_graph(const void *kern, const TeamPlan &plan, void **params,
+                 cudaGraphConditionalHandle *more, void *zero, size_t zero_bytes, unsigned *ctl,
+                 cudaGraph_t *graph) {
+  cudaGraph_t g = nullptr;
+  if (cudaGraphCreate(&g, 0) != cudaSuccess) return SFR_CUDA_ERROR;
+  *graph = g;
+  if (cudaGraphConditionalHandleCreate(more, g, 1, cudaGraphCondAssignDefault) != cudaSuccess)
+    return SFR_CUDA_ERROR;
+  cudaGraphNode_t prev = nullptr;
+  const std::pair<void *, size_t> clear[] = {{zero, zero_bytes}, {ctl, 64}};
+  for (const auto &c : clear) {
+    cudaMemsetParams mp{};
+    mp.dst = c.first;
+    mp.elementSize = 4;
+    mp.width = c.second / 4;
+    mp.height = 1;
+    cudaGraphNode_t node = nullptr;
+    if (cudaGraphAddMemsetNode(&node, g, prev ? &prev : nullptr, prev ? 1 : 0, &mp) != cudaSuccess)
+      return SFR_CUDA_ERROR;
+    prev = node;
+  }
+  cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
+  cp.conditional.handle = *more;
+  cp.conditional.type = cudaGraphCondTypeWhile;
+  cp.conditional.size = 1;
+  cudaGraphNode_t loop = nullptr;
+  if (cudaGraphAddNode(&loop, g, &prev, 1, &cp) != cudaSuccess) return SFR_CUDA_ERROR;
+  cudaKernelNodeParams kp{};
+  kp.func = const_cast<void *>(kern);
+  kp.gridDim = dim3(plan.grid);
+  kp.blockDim = dim3(plan.shape.threads);
+  kp.sharedMemBytes = static_cast<unsigned>(plan.shape.smem);
+  kp.kernelParams = params;  // the values are copied
+  cudaGraphNode_t kn = nullptr;
+  if (cudaGraphAddKernelNode(&kn, cp.conditional.phGraph_out[0], nullptr, 0, &kp) != cudaSuccess)
+    return SFR_CUDA_ERROR;
+  cudaKernelNodeAttrValue coop{};
+  coop.cooperative = 1;
+  return cudaGraphKernelNodeSetAttribute(kn, cudaLaunchAttributeCooperative, &coop) == cudaSuccess
+             ? SFR_OK
+             : SFR_CUDA_ERROR;
+}
+
 }  // namespace sfr
 
 extern "C" {
@@ -371,8 +508,8 @@ int sfr_gpu_batch_create(int32_t nsys, const int32_t *neq, const int32_t *nad,
     slices += h.nslices;
     src += ns;
     if (rows > INT32_MAX || src > INT32_MAX || cat.sptr.back() < 0) return SFR_BAD_INPUT;
-    // default work estimate: slices x an iteration count growing like n^(1/3)
-    b->weight.push_back(static_cast<double>(h.nslices) * std::cbrt(static_cast<double>(neq[s])));
+    // default work estimate: slices x iterations, about 15 n^(1/3) of them
+    b->weight.push_back(15.0 * h.nslices * std::cbrt(static_cast<double>(neq[s])));
   }
   b->team_ms.assign(nsys, 0.0);
   cat.n = static_cast<int32_t>(rows);
@@ -395,6 +532,7 @@ int sfr_gpu_batch_create(int32_t nsys, const int32_t *neq, const int32_t *nad,
       cudaMalloc(&b->d_b, sizeof(double) * nrow) != cudaSuccess ||
       cudaMalloc(&b->d_x, sizeof(double) * nrow) != cudaSuccess ||
       cudaMalloc(&b->d_bar, sizeof(unsigned) * 2 * nsys) != cudaSuccess ||
+      cudaMalloc(&b->d_systems, sizeof(int4) * nsys) != cudaSuccess ||
       cudaMalloc(&b->d_out, sizeof(sfr::SolveOut) * nsys) != cudaSuccess ||
       cudaMalloc(&b->d_ctl, 64) != cudaSuccess)
     return SFR_CUDA_ERROR;
@@ -708,6 +846,7 @@ int sfr_gpu_batch_destroy(sfr_batch *b) {
   if (b->cat.stream) cudaStreamDestroy(b->cat.stream);
   cudaFree(b->d_block);
   cudaFree(b->d_sys);
+  cudaFree(b->d_systems);
   cudaFree(b->d_bar);
   cudaFree(b->ws);
   cudaFree(b->d_out);

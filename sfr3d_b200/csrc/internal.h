@@ -147,15 +147,6 @@ int enqueue_team_mixed(sfr_system *s, int32_t solver, const double *d_b, double 
                        uint32_t maxit, int32_t newx, const TeamTable &team, int grid, void *ws,
                        SolveOut *d_out, unsigned *ctl, cudaStream_t st);
 
-// The on-chip engine's team launch (onchip.cu): FP64 PCG.  A block takes at
-// most team_max_slices_onchip slices.
-size_t team_ws_bytes_onchip(int n, int grid);
-int team_max_grid_onchip(int device);
-int team_max_slices_onchip(int device);
-int enqueue_team_onchip(sfr_system *s, const double *d_b, double *d_x, double tol, uint32_t maxit,
-                        int32_t newx, const TeamTable &team, int grid, void *ws, SolveOut *d_out,
-                        unsigned *ctl, cudaStream_t st);
-
 // Resident engine (resident.cu): mixed PCG, one right-hand side, the
 // system's own diagonal.  resident_fits: the pattern and size allow it;
 // solve_resident returns SFR_UNSUPPORTED when the diagonal is not positive.

@@ -38,16 +38,14 @@
 #include "common.cuh"
 #include "internal.h"
 #include "persist.cuh"
+#include "team_plan.h"
+#include "team_sync.cuh"
 
 namespace sfr {
 
 namespace {
 
 constexpr int kChunk = 6;  // slots of a row loaded before their gathers (a hex cell's faces)
-
-struct alignas(64) ChipSlot {
-  ulonglong2 v[4];  // {value, epoch}
-};
 
 struct ChipArgs {
   int n, nslices;
@@ -57,61 +55,12 @@ struct ChipArgs {
   double *x;
   double *p;        // grid form: the search direction, nslices * 32 entries
   double *z;        // grid form, level 0: M r, nslices * 32 entries
-  ChipSlot *slots;  // grid form: two buffers of one slot a block, zero at launch
-  unsigned *ticks;  // grid form: 16 words a block, zero at launch
-  int *err;
-  unsigned spin_limit;
+  TeamSync sync;    // grid form
   SolveOut *out;
   double tol;
   unsigned maxit;
   int newx;
 };
-
-// The blocks that solve one system together, and this block's part: slices
-// [s0, s1) of the system's [first, first + count), which the team's blocks
-// [b0, b1) share in order.  A launch for one system is one team.
-struct ChipTeam {
-  int s0, s1, first, count, b0, b1;
-  int row_end;  // the system's rows end here
-  int sys;
-  unsigned long long t0;  // the block's start (global_ns)
-  __device__ __forceinline__ int owner(int row) const {
-    const long long B = b1 - b0, ns = count, sl = row / kWarp - first;
-    return b0 + static_cast<int>(((sl + 1) * B + ns - 1) / ns - 1);
-  }
-};
-
-// Four values summed over a warp with six 64-bit shuffles (a butterfly that
-// halves the values a lane carries before it halves the lanes): lane l ends
-// with the total of value l >> 3, the same bits in all eight of its lanes.
-__device__ __forceinline__ double warp_sum4(const double (&v)[4]) {
-  const int lane = threadIdx.x & 31;
-  const bool h16 = lane & 16, h8 = lane & 8;
-  const double a0 = (h16 ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16);
-  const double a1 = (h16 ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16);
-  double t = (h8 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, h8 ? a0 : a1, 8);
-  t += __shfl_xor_sync(0xffffffffu, t, 4);
-  t += __shfl_xor_sync(0xffffffffu, t, 2);
-  t += __shfl_xor_sync(0xffffffffu, t, 1);
-  return t;
-}
-
-// The block's totals of four values: lanes 0, 8, 16, 24 of warp 0 hold value
-// 0, 1, 2, 3 (other threads: unspecified).  sm: 4 * 32 doubles.
-__device__ __forceinline__ double block_sum4(const double (&v)[4], double *sm) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const double t = warp_sum4(v);
-  if ((lane & 7) == 0) sm[(lane >> 3) * 32 + warp] = t;
-  __syncthreads();
-  double s = 0.0;
-  if (warp == 0) {
-    double w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = lane < nw ? sm[i * 32 + lane] : 0.0;
-    s = warp_sum4(w);
-  }
-  return s;
-}
 
 // The scalars of iteration j from the exchanged products {mu, delta, gamma,
 // nu}: false when the solve stops (status and iters set).  Iteration j - 1's
@@ -172,133 +121,6 @@ __device__ __forceinline__ void put_result(SolveOut *out, const Scalars &sc,
   *out = o;
 }
 
-// ---- grid form: synchronisation through L2 -------------------------------
-
-// {value, epoch} in one 16-byte word, stored and loaded whole.
-__device__ __forceinline__ void st_slot(ulonglong2 *p, double v, unsigned long long epoch) {
-  asm volatile(
-      "{\n .reg .b128 t;\n mov.b128 t, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], t;\n}" ::"l"(p),
-      "l"(__double_as_longlong(v)), "l"(epoch)
-      : "memory");
-}
-__device__ __forceinline__ bool ld_slot(const ulonglong2 *p, double *v, unsigned long long epoch) {
-  unsigned long long lo, hi;
-  asm volatile(
-      "{\n .reg .b128 t;\n ld.relaxed.gpu.global.b128 t, [%2];\n mov.b128 {%0, %1}, t;\n}"
-      : "=l"(lo), "=l"(hi)
-      : "l"(p)
-      : "memory");
-  *v = __longlong_as_double(static_cast<long long>(lo));
-  return hi == epoch;
-}
-
-// Totals of four values over the team, in every thread, the same bits in all
-// its blocks.  Each block writes its totals with the epoch beside each value;
-// thread b of every block polls block b's slot, so the values arrive with
-// the poll: one L2 round trip.  Two buffers alternate: a block writes epoch e
-// only after it read every block's epoch e - 1, which each published after it
-// had read every epoch e - 2.  kFence: every global write before the call, in
-// any block, is visible after it in all.  Bounded: after spin_limit polls a
-// block records SFR_TIMEOUT in *err, and a block that sees *err set stops
-// waiting.  False on either.  sm: 32 * 4 + 4 doubles, bad: a shared word.
-template <bool kFence>
-__device__ __forceinline__ bool grid_sum4(const ChipArgs &a, const ChipTeam &t, unsigned &epoch,
-                                          const double (&acc)[4], double (&tot)[4], double *sm,
-                                          int *bad) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int G = t.b1 - t.b0;
-  ++epoch;
-  const double s = block_sum4(acc, sm);
-  if (G == 1) {  // a team of one block: no other block to tell
-    if (warp == 0 && (lane & 7) == 0) sm[(lane >> 3) * 32] = s;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) tot[i] = sm[i * 32];
-    __syncthreads();
-    return true;
-  }
-  ChipSlot *cur = a.slots + static_cast<size_t>(epoch & 1u) * gridDim.x + t.b0;
-  if (warp == 0 && (lane & 7) == 0) {
-    if (kFence) cuda::atomic_thread_fence(cuda::memory_order_release, cuda::thread_scope_device);
-    st_slot(&cur[blockIdx.x - t.b0].v[lane >> 3], s, epoch);
-  }
-  if (threadIdx.x == 0) *bad = 0;
-  __syncthreads();  // sm is free again; *bad is 0
-  const int watchers = min(static_cast<int>(blockDim.x), (G + 31) & ~31);
-  if (static_cast<int>(threadIdx.x) < watchers) {
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
-    cuda::atomic_ref<int, cuda::thread_scope_device> err(*a.err);
-    for (int b = threadIdx.x; b < G; b += watchers) {
-      double w[4];
-      for (unsigned spins = 0;; ++spins) {
-        bool all = true;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) all &= ld_slot(&cur[b].v[i], &w[i], epoch);
-        if (all) break;
-        if ((spins & 63u) == 63u && err.load(cuda::memory_order_relaxed) != 0) {
-          *bad = 1;
-          break;
-        }
-        if (spins > a.spin_limit) {
-          int expected = 0;
-          err.compare_exchange_strong(expected, SFR_TIMEOUT, cuda::memory_order_relaxed);
-          *bad = 1;
-          break;
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] += w[i];
-    }
-    __syncwarp();
-    if (kFence) cuda::atomic_thread_fence(cuda::memory_order_acquire, cuda::thread_scope_device);
-    const double q = warp_sum4(v);
-    if ((lane & 7) == 0) sm[(lane >> 3) * 32 + warp] = q;
-  }
-  __syncthreads();
-  const int ww = watchers >> 5;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    double q = sm[i * 32];
-    for (int w = 1; w < ww; ++w) q += sm[i * 32 + w];
-    tot[i] = q;
-  }
-  const bool ok = *bad == 0;
-  __syncthreads();
-  return ok;
-}
-
-// The blocks [range[0], range[1]] owning the columns this block gathers from.
-template <typename I>
-__device__ __forceinline__ void gather_range(const ChipTeam &t, const int *sm_sp, const I *cols,
-                                             int *range) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  int cmin = t.s0 * kWarp, cmax = t.s1 * kWarp - 1;
-  for (int s = t.s0 + warp; s < t.s1; s += nw) {
-    const int row = s * kWarp + lane;
-    if (row >= t.row_end) continue;  // padding: its columns mean nothing
-    for (int e = sm_sp[s - t.s0] + lane; e < sm_sp[s - t.s0 + 1]; e += kWarp) {
-      const int c = slot_col(cols, e, row);
-      cmin = min(cmin, c);
-      cmax = max(cmax, c);
-    }
-  }
-  if (threadIdx.x == 0) {
-    range[0] = cmin;
-    range[1] = cmax;
-  }
-  __syncthreads();
-  atomicMin(range, cmin);
-  atomicMax(range + 1, cmax);
-  __syncthreads();
-  const int lo = t.owner(range[0]), hi = t.owner(range[1]);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    range[0] = lo;
-    range[1] = hi;
-  }
-  __syncthreads();
-}
-
 // Where a block of the grid form keeps its rows' state, by what fits:
 //   level 0  M q in shared memory (8 B a row); z, x, ad and p in L2 or HBM
 //   level 1  also z (16 B a row)
@@ -312,7 +134,11 @@ constexpr int kLevels = 4;
 __host__ __device__ constexpr int level_bytes(int level) {
   return level == 0 ? 8 : level == 1 ? 16 : level == 2 ? 24 : 40;
 }
-enum Slots { kHold, kKeep, kStream };
+enum Slots { kHold, kKeep, kStream, kPolicy };  // kPolicy: kKeep or kStream, by the call
+
+// A batch's slices (of 6 slots: 1.9 KB) up to which kPolicy keeps the slots:
+// 70 MB, the line kKeepBytes draws for one system.
+constexpr int kKeepSlices = 36000;
 
 // Threads a block: 24 warps at 80 registers hold a slice's slots, gathers and
 // the four sums without spilling.  An iteration at 96^3 / 128^3: 13.2 / 41.1
@@ -320,15 +146,23 @@ enum Slots { kHold, kKeep, kStream };
 // 17.3 / 51.5.
 constexpr int kGridThreads = 768;
 
-// A block's static shared memory.
-struct GridShared {
-  double red[32 * 4];
-  int bad, range[2];
+// Where a system of a batched launch stands between two rounds (z, x and p
+// are in a.z, a.x and a.p).
+struct ChipState {
+  double conv, nu_old;
+  unsigned j;
+  unsigned long long t0;  // its first round's start (global_ns)
 };
 
+// The solve, or (st given) at most `cap` of its iterations, going on from
+// *st when `resume`; true when it is over.  epoch and tick: what the team's
+// exchanges and publications count from.
 template <typename I, int kLevel, Slots kSlots>
-__device__ __forceinline__ void pcg_grid_body(const ChipArgs &a, const ChipTeam &t,
-                                              double *sm_dyn, GridShared &sh) {
+__device__ __forceinline__ bool pcg_grid_body(const ChipArgs &a, const TeamPart &t,
+                                              double *sm_dyn, TeamShared &sh, unsigned epoch,
+                                              unsigned tick, ChipState *st,
+                                              const RoundTable *rt, bool resume,
+                                              unsigned cap) {
   double *const red = sh.red;
   int *const bad = &sh.bad, *const range = sh.range;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
@@ -354,7 +188,13 @@ __device__ __forceinline__ void pcg_grid_body(const ChipArgs &a, const ChipTeam 
   const bool alone = t.b1 - t.b0 == 1;
   if (!alone) gather_range(t, sm_sp, cols, range);
 
-  unsigned epoch = 0, tick = 0;
+  uint64_t pol = 0;
+  if (kSlots == kPolicy) {
+    if (t.slices_left > kKeepSlices)
+      asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+    else
+      asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+  }
   double acc[4], tot[4];
 
   // y = A v for the block's rows, v in a.p (own rows also in sm_p): post(lr,
@@ -391,9 +231,13 @@ __device__ __forceinline__ void pcg_grid_body(const ChipArgs &a, const ChipTeam 
           for (int u = 0; u < kChunk; ++u)
             if (e0 + u < w) {
               const int k = (e0 + u) * kWarp;
-              const int o = kSlots == kStream ? __ldcs(c + k) : __ldcg(c + k);
+              const int o = kSlots == kPolicy   ? ld_mat(c + k, pol)
+                            : kSlots == kStream ? __ldcs(c + k)
+                                                : __ldcg(c + k);
               jj[u] = sizeof(I) == 2 ? row + o : o;
-              vv[u] = kSlots == kStream ? __ldcs(v + k) : __ldcg(v + k);
+              vv[u] = kSlots == kPolicy   ? ld_mat(v + k, pol)
+                      : kSlots == kStream ? __ldcs(v + k)
+                                          : __ldcg(v + k);
             }
         };
         load(0);
@@ -419,33 +263,52 @@ __device__ __forceinline__ void pcg_grid_body(const ChipArgs &a, const ChipTeam 
       __syncthreads();
       return true;
     }
-    return neighbour_wait(a.ticks, a.err, a.spin_limit, ++tick, range[0], range[1]);
+    return neighbour_wait(a.sync.ticks, a.sync.err, a.sync.spin_limit, ++tick, range[0], range[1]);
   };
 
-  // x0 and (b, M b); p = z = M b, or p = x0 for the product with the start
-  acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
-  for (int lr = threadIdx.x; lr < own; lr += blockDim.x) {
-    const double d = __ldcg(a.diag + r0 + lr), b = ld_vec(a.b + r0 + lr);
-    const double z = xdiv(b, d);
-    acc[0] += b * z;
-    const double x0 = a.newx ? 0.0 : ld_vec(a.x + r0 + lr);
-    if (kLevel >= 2 || a.newx) vx[lr] = x0;
-    if (kLevel == 3) sm_d[lr] = d;
-    vz[lr] = z;
-    put_p(lr, a.newx ? z : x0);
-  }
-  if (!grid_sum4<true>(a, t, epoch, acc, tot, red, bad)) return;
-  Scalars sc(a.tol * sqrt(fabs(tot[0])));
-  if (!a.newx) {
-    matvec([&](int lr, double y, double, double d, double) {
-      vz[lr] = xdiv(xsub(ld_vec(a.b + r0 + lr), y), d);
-    });
-    if (!grid_sum4<false>(a, t, epoch, acc, tot, red, bad)) return;  // every gather of x0 is done
-    for (int lr = threadIdx.x; lr < own; lr += blockDim.x) put_p(lr, vz[lr]);
-    if (!publish()) return;
+  Scalars sc(0.0);
+  unsigned j = 0;
+  if (!resume) {
+    // x0 and (b, M b); p = z = M b, or p = x0 for the product with the start
+    acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
+    for (int lr = threadIdx.x; lr < own; lr += blockDim.x) {
+      const double d = __ldcg(a.diag + r0 + lr), b = ld_vec(a.b + r0 + lr);
+      const double z = xdiv(b, d);
+      acc[0] += b * z;
+      const double x0 = a.newx ? 0.0 : ld_vec(a.x + r0 + lr);
+      if (kLevel >= 2 || a.newx) vx[lr] = x0;
+      if (kLevel == 3) sm_d[lr] = d;
+      vz[lr] = z;
+      put_p(lr, a.newx ? z : x0);
+    }
+    if (!team_sum<4, true>(a.sync, t, epoch, acc, tot, red, bad)) return false;
+    sc = Scalars(a.tol * sqrt(fabs(tot[0])));
+    if (!a.newx) {
+      matvec([&](int lr, double y, double, double d, double) {
+        vz[lr] = xdiv(xsub(ld_vec(a.b + r0 + lr), y), d);
+      });
+      // every gather of x0 is done
+      if (!team_sum<4, false>(a.sync, t, epoch, acc, tot, red, bad)) return false;
+      for (int lr = threadIdx.x; lr < own; lr += blockDim.x) put_p(lr, vz[lr]);
+      if (!publish()) return false;
+    }
+  } else {
+    sc = Scalars(__ldcg(&st->conv));
+    sc.nu_old = __ldcg(&st->nu_old);
+    j = __ldcg(&st->j);
+    for (int lr = threadIdx.x; lr < own; lr += blockDim.x) {
+      if (kLevel >= 1) vz[lr] = ld_vec(a.z + r0 + lr);
+      if (kLevel >= 2) vx[lr] = ld_vec(a.x + r0 + lr);
+      if (kLevel == 3) {
+        sm_d[lr] = __ldcg(a.diag + r0 + lr);
+        sm_p[lr] = ld_vec(a.p + r0 + lr);
+      }
+    }
+    __syncthreads();
   }
 
-  for (unsigned j = 0;; ++j) {
+  const unsigned stop = j + min(cap, 0xffffffffu - j);
+  for (;; ++j) {
     acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
     matvec([&](int lr, double y, double p, double d, double z) {
       const double mq = xdiv(y, d);
@@ -455,7 +318,7 @@ __device__ __forceinline__ void pcg_grid_body(const ChipArgs &a, const ChipTeam 
       acc[2] += y * mq;
       acc[3] += (d * z) * z;
     });
-    if (!grid_sum4<false>(a, t, epoch, acc, tot, red, bad)) return;
+    if (!team_sum<4, false>(a.sync, t, epoch, acc, tot, red, bad)) return false;
     if (!sc.next(tot, j, a.maxit)) break;
     const double alpha = sc.alpha, beta = sc.beta;
     for (int lr = threadIdx.x; lr < own; lr += blockDim.x) {
@@ -465,7 +328,21 @@ __device__ __forceinline__ void pcg_grid_body(const ChipArgs &a, const ChipTeam 
       vx[lr] = xadd(vx[lr], xmul(alpha, p));
       put_p(lr, xadd(z, xmul(beta, p)));
     }
-    if (!publish()) return;
+    if (!publish()) return false;
+    if (st && j + 1 == stop) {  // the round is over: the state goes to global memory
+      for (int lr = threadIdx.x; lr < own; lr += blockDim.x) {
+        if (kLevel >= 1) st_vec(a.z + r0 + lr, vz[lr]);
+        if (kLevel >= 2) st_vec(a.x + r0 + lr, vx[lr]);
+      }
+      if (static_cast<int>(blockIdx.x) == t.b0 && threadIdx.x == 0) {
+        st->conv = sc.conv;
+        st->nu_old = sc.nu_old;
+        st->j = j + 1;
+        if (!resume) st->t0 = t.t0;
+        rt->iters[t.sys] = static_cast<int>(j + 1);
+      }
+      return false;
+    }
   }
 
   // xKx, ||x||, ||b - Ax||_M, ||b - Ax||  (Cg.c:155-176), with x in p's place
@@ -474,7 +351,7 @@ __device__ __forceinline__ void pcg_grid_body(const ChipArgs &a, const ChipTeam 
     if (kLevel >= 2) st_vec(a.x + r0 + lr, x);
     put_p(lr, x);
   }
-  if (!publish()) return;
+  if (!publish()) return false;
   acc[0] = acc[1] = acc[2] = acc[3] = 0.0;
   matvec([&](int lr, double y, double x, double d, double) {
     const double r = xsub(ld_vec(a.b + r0 + lr), y);
@@ -483,57 +360,63 @@ __device__ __forceinline__ void pcg_grid_body(const ChipArgs &a, const ChipTeam 
     acc[2] += r * xdiv(r, d);
     acc[3] += r * r;
   });
-  if (!grid_sum4<false>(a, t, epoch, acc, tot, red, bad)) return;
+  if (!team_sum<4, false>(a.sync, t, epoch, acc, tot, red, bad)) return false;
   if (static_cast<int>(blockIdx.x) == t.b0 && threadIdx.x == 0)
-    put_result(a.out + t.sys, sc, tot, (global_ns() - t.t0) * 1e-6);
+    put_result(a.out + t.sys, sc, tot, (global_ns() - (resume ? st->t0 : t.t0)) * 1e-6);
+  return true;
 }
 
 // One system over the whole grid.
 template <typename I, int kLevel, Slots kSlots>
 __global__ void __launch_bounds__(kGridThreads, 1) pcg_grid_kernel(const ChipArgs a) {
   extern __shared__ double sm_dyn[];
-  __shared__ GridShared sh;
-  ChipTeam t{};
+  __shared__ TeamShared sh;
+  TeamPart t{};
   block_slices(a.nslices, &t.s0, &t.s1);
   t.count = a.nslices;
   t.b1 = gridDim.x;
   t.row_end = a.n;
   t.t0 = global_ns();
-  pcg_grid_body<I, kLevel, kSlots>(a, t, sm_dyn, sh);
+  (void)pcg_grid_body<I, kLevel, kSlots>(a, t, sm_dyn, sh, 0u, 0u, nullptr, nullptr, false,
+                                          0xffffffffu);
 }
 
-// Many systems, a team of blocks each (batched.cu's table).  A block picks
-// its level by its own rows: blocks of one team need not agree, they only
-// exchange sums and p.  Two blocks an SM: twice the teams, and a small
-// system's share is a finer one.
-constexpr int kTeamThreads = 384;
+// Many systems, a team of blocks each, in rounds (team_sync.cuh).  A block
+// picks its level by its own rows: blocks of one team need not agree, they
+// only exchange sums and p.
 
-template <typename I>
-__global__ void __launch_bounds__(kTeamThreads, 2) pcg_team_kernel(const ChipArgs a,
-                                                                   const TeamTable tt, int smem) {
+template <typename I, int kT>
+__global__ void __launch_bounds__(kT, kGridThreads / kT)
+    pcg_team_kernel(const ChipArgs a, const TeamTable tt, const RoundTable rt, ChipState *states,
+                    int smem) {
   extern __shared__ double sm_dyn[];
-  __shared__ GridShared sh;
-  const int4 e = tt.block[blockIdx.x];
-  const int2 y = tt.sys[blockIdx.x];
-  ChipTeam t;
-  t.s0 = e.x;
-  t.s1 = e.y;
-  t.b0 = e.z;
-  t.b1 = e.w;
-  t.first = tt.block[e.z].x;
-  t.count = tt.block[e.w - 1].y - t.first;
-  t.sys = y.x;
-  t.row_end = y.y;
-  t.t0 = global_ns();
-  const int slices = t.s1 - t.s0, rows = slices * kWarp;
-  const int left = smem - 4 * (slices + 1);
-  const int slots = a.sptr[t.s1] - a.sptr[t.s0];
-  if (rows * level_bytes(3) + slots * static_cast<int>(8 + sizeof(I)) <= left)
-    pcg_grid_body<I, 3, kHold>(a, t, sm_dyn, sh);
-  else if (rows * level_bytes(2) <= left)
-    pcg_grid_body<I, 2, kKeep>(a, t, sm_dyn, sh);
-  else
-    pcg_grid_body<I, 0, kKeep>(a, t, sm_dyn, sh);
+  __shared__ TeamShared sh;
+  const unsigned round = __ldcg(rt.ctl);
+  {
+    const TeamPart mine = team_part(tt, rt, round, sh.scan);
+    if (threadIdx.x == 0) sh.part = mine;
+    __syncthreads();
+  }
+  const TeamPart &t = sh.part;
+  bool over = false;
+  if (t.b1 > t.b0) {
+    const unsigned base = round_base(round), cap = round_cap(rt, t, round);
+    ChipState *st = states + t.sys;
+    const int slices = t.s1 - t.s0, rows = slices * kWarp;
+    const int left = smem - 4 * (slices + 1);
+    const int slots = __ldg(a.sptr + t.s1) - __ldg(a.sptr + t.s0);
+    if (rows * level_bytes(3) + slots * static_cast<int>(8 + sizeof(I)) <= left)
+      over = pcg_grid_body<I, 3, kHold>(a, t, sm_dyn, sh, base, base, st, &rt,
+                                        round > 0, cap);
+    else if (rows * level_bytes(2) <= left)
+      over = pcg_grid_body<I, 2, kPolicy>(a, t, sm_dyn, sh, base, base, st, &rt,
+                                        round > 0, cap);
+    else
+      over = pcg_grid_body<I, 0, kPolicy>(a, t, sm_dyn, sh, base, base, st, &rt,
+                                        round > 0, cap);
+  }
+  __syncthreads();
+  end_round(rt, over && static_cast<int>(blockIdx.x) == t.b0, t.sys);
 }
 
 // ---- cluster form --------------------------------------------------------
@@ -568,7 +451,7 @@ __device__ __forceinline__ void cluster_sum4(double *ex, unsigned &buf, const do
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   buf ^= 1u;
   double *cur = ex + buf * (kMaxCluster * 4);
-  const double s = block_sum4(acc, sm);
+  const double s = block_sum_n<4>(acc, sm);
   if (warp == 0) {
     // lane l holds value l >> 3; it stores it into ranks l & 7 and 8 + (l & 7)
     const unsigned dst = smem_u32(cur + blockIdx.x * 4 + (lane >> 3));
@@ -765,7 +648,7 @@ int smem_optin(int device) {
 }
 
 // static shared memory of the kernels (reductions, exchange buffers), rounded up
-constexpr size_t kGridStatic = 1280, kClusterStatic = 2304;
+constexpr size_t kGridStatic = 1536, kClusterStatic = 2304;
 
 struct Shape {
   const void *kern = nullptr;
@@ -892,55 +775,41 @@ bool grid_shape(const sfr_system *s, Shape *sh) {
   return true;
 }
 
-// Dynamic shared memory of a team block: two to an SM.
-size_t team_smem(int device) {
-  int per_sm = 0;
-  if (cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) !=
-      cudaSuccess)
-    return 0;
-  // a block also takes its static shared memory and the system's 1 KB
-  const int half = per_sm / 2 - 1024 - static_cast<int>(kGridStatic);
-  return half > 0 ? static_cast<size_t>(half) / 256 * 256 : 0;
-}
-
 size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
+
+const void *team_kernel(const sfr_system *s, int per_sm) {
+  if (per_sm == 1)
+    return s->A.off ? reinterpret_cast<const void *>(pcg_team_kernel<int16_t, kGridThreads>)
+                    : reinterpret_cast<const void *>(pcg_team_kernel<int, kGridThreads>);
+  return s->A.off ? reinterpret_cast<const void *>(pcg_team_kernel<int16_t, kGridThreads / 2>)
+                  : reinterpret_cast<const void *>(pcg_team_kernel<int, kGridThreads / 2>);
+}
 
 }  // namespace
 
-int team_max_slices_onchip(int device) {
-  const size_t b = team_smem(device);
-  return b ? static_cast<int>((b - 8) / (kWarp * level_bytes(0) + 4)) : 0;
+// The model: 16 boxes of 16^3 on 9 blocks each (14 slices a block) 5.5 us an
+// iteration, 32^3 (111 slices) 11.0, 48^3 (375) 36.8; a block alone with 16
+// slices 2.4.
+TeamShape team_shape_onchip(const sfr_system *s, int per_sm) {
+  return team_shape(s->device, team_kernel(s, per_sm), kGridThreads / per_sm, per_sm,
+                    kWarp * level_bytes(0) + 4, TeamModel{0.9f, 4.5f, 0.1f});
 }
 
-int team_max_grid_onchip(int device) {
-  const size_t b = team_smem(device);
-  int occ = INT32_MAX;
-  for (const void *k : {reinterpret_cast<const void *>(pcg_team_kernel<int16_t>),
-                        reinterpret_cast<const void *>(pcg_team_kernel<int>)}) {
-    int o = 0;
-    if (!b ||
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             static_cast<int>(b)) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, k, kTeamThreads, b) != cudaSuccess)
-      return 0;
-    occ = std::min(occ, o);
-  }
-  // neighbour_wait watches one block a thread
-  return std::min(kTeamThreads, occ * num_sms(device));
-}
-
-size_t team_ws_bytes_onchip(int n, int grid) {
-  return 2 * align256(sizeof(double) * static_cast<size_t>(n)) +
-         align256(sizeof(ChipSlot) * 2 * static_cast<size_t>(grid)) +
+size_t team_ws_bytes_onchip(int n, int grid, int nsys) {
+  return align256((sizeof(ChipState) + 2 * sizeof(int)) * static_cast<size_t>(nsys)) +
+         2 * align256(sizeof(double) * static_cast<size_t>(n)) +
+         align256(sizeof(TeamSlot) * 2 * static_cast<size_t>(grid)) +
          align256(64 * static_cast<size_t>(grid));
 }
 
-int enqueue_team_onchip(sfr_system *s, const double *d_b, double *d_x, double tol, uint32_t maxit,
-                        int32_t newx, const TeamTable &team, int grid, void *ws, SolveOut *d_out,
-                        unsigned *ctl, cudaStream_t st) {
+int graph_team_onchip(sfr_system *s, const double *d_b, double *d_x, double tol, uint32_t maxit,
+                      int32_t newx, const TeamPlan &plan, void *ws, SolveOut *d_out,
+                      unsigned *ctl, cudaGraph_t *graph) {
   const size_t vec = align256(sizeof(double) * static_cast<size_t>(s->n));
-  const size_t slot_b = align256(sizeof(ChipSlot) * 2 * static_cast<size_t>(grid));
-  const size_t tick_b = align256(64 * static_cast<size_t>(grid));
+  const size_t slot_b = align256(sizeof(TeamSlot) * 2 * static_cast<size_t>(plan.grid));
+  const size_t tick_b = align256(64 * static_cast<size_t>(plan.grid));
+  const size_t state_b =
+      align256((sizeof(ChipState) + 2 * sizeof(int)) * static_cast<size_t>(plan.nsys));
   char *base = static_cast<char *>(ws);
   ChipArgs a{};
   a.n = s->n;
@@ -952,28 +821,23 @@ int enqueue_team_onchip(sfr_system *s, const double *d_b, double *d_x, double to
   a.diag = s->d_diag;
   a.b = d_b;
   a.x = d_x;
-  a.slots = reinterpret_cast<ChipSlot *>(base);
-  a.ticks = reinterpret_cast<unsigned *>(base + slot_b);
-  a.p = reinterpret_cast<double *>(base + slot_b + tick_b);
-  a.z = reinterpret_cast<double *>(base + slot_b + tick_b + vec);
-  a.err = reinterpret_cast<int *>(ctl + 2);
-  a.spin_limit = 1u << 22;
+  a.sync.slots = reinterpret_cast<TeamSlot *>(base);
+  a.sync.ticks = reinterpret_cast<unsigned *>(base + slot_b);
+  a.sync.err = reinterpret_cast<int *>(ctl + 2);
+  a.sync.spin_limit = 1u << 22;
+  ChipState *states = reinterpret_cast<ChipState *>(base + slot_b + tick_b);
+  RoundTable rt = round_table(plan, reinterpret_cast<int *>(states + plan.nsys), ctl);
+  a.p = reinterpret_cast<double *>(base + slot_b + tick_b + state_b);
+  a.z = reinterpret_cast<double *>(base + slot_b + tick_b + state_b + vec);
   a.out = d_out;
   a.tol = tol;
   a.maxit = maxit;
   a.newx = newx;
-  if (cudaMemsetAsync(base, 0, slot_b + tick_b, st) != cudaSuccess ||
-      cudaMemsetAsync(ctl, 0, 64, st) != cudaSuccess)
-    return SFR_CUDA_ERROR;
-  int smem = static_cast<int>(team_smem(s->device));
-  TeamTable tt = team;
-  void *params[] = {&a, &tt, &smem};
-  const void *k = s->A.off ? reinterpret_cast<const void *>(pcg_team_kernel<int16_t>)
-                           : reinterpret_cast<const void *>(pcg_team_kernel<int>);
-  return cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kTeamThreads), params,
-                                     static_cast<size_t>(smem), st) == cudaSuccess
-             ? SFR_OK
-             : SFR_CUDA_ERROR;
+  int smem = static_cast<int>(plan.shape.smem);
+  TeamTable tt = plan.table;
+  void *params[] = {&a, &tt, &rt, &states, &smem};
+  return rounds_graph(team_kernel(s, plan.shape.per_sm), plan, params, &rt.more, base,
+                      slot_b + tick_b + state_b, ctl, graph);
 }
 
 int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double *d_x, double tol,
@@ -987,7 +851,7 @@ int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double 
 
   auto align = [](size_t v) { return (v + 255) & ~static_cast<size_t>(255); };
   const size_t vec = align(sizeof(double) * static_cast<size_t>(s->A.nslices) * kWarp);
-  const size_t slot_b = align(sizeof(ChipSlot) * 2 * static_cast<size_t>(sh.grid));
+  const size_t slot_b = align(sizeof(TeamSlot) * 2 * static_cast<size_t>(sh.grid));
   const size_t tick_b = align(64 * static_cast<size_t>(sh.grid)) + 256;  // + the error word
   const size_t out_b = align(sizeof(SolveOut));
   // x is written while b is still read: a caller's x that overlaps b gets a
@@ -1013,7 +877,7 @@ int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double 
   a.tol = tol;
   a.maxit = maxit;
   a.newx = newx;
-  a.spin_limit = 1u << 22;
+  a.sync.spin_limit = 1u << 22;
   SolveOut *dev_out = reinterpret_cast<SolveOut *>(base);
   base += out_b;
   if (overlap) {
@@ -1023,9 +887,9 @@ int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double 
     base += vec;
   }
   if (!sh.cluster) {
-    a.slots = reinterpret_cast<ChipSlot *>(base);
-    a.ticks = reinterpret_cast<unsigned *>(base + slot_b);
-    a.err = reinterpret_cast<int *>(base + slot_b + tick_b - 256);
+    a.sync.slots = reinterpret_cast<TeamSlot *>(base);
+    a.sync.ticks = reinterpret_cast<unsigned *>(base + slot_b);
+    a.sync.err = reinterpret_cast<int *>(base + slot_b + tick_b - 256);
     a.p = reinterpret_cast<double *>(base + slot_b + tick_b);
     a.z = reinterpret_cast<double *>(base + slot_b + tick_b + vec);
     if (cudaMemsetAsync(base, 0, slot_b + tick_b, st) != cudaSuccess) return SFR_CUDA_ERROR;

@@ -224,3 +224,39 @@ def test_team_launch_with_wide_columns(cuda):
         assert info.status == sv.OK and abs(info.iters - ref.iters) <= 1
         assert rel(x, ref.x) < BAR
     g.close()
+
+
+@pytest.mark.parametrize("precision", [sv.FP64, sv.MIXED], ids=["fp64", "mixed"])
+def test_rounds_of_a_team_launch(cuda, precision):
+    """Anisotropic boxes that take far more iterations than their size
+    suggests, beside cubes that take fewer: several rounds, with the blocks
+    shared out anew between them.  FP64 at the FP64 bar; mixed meets the
+    reference's criterion on the FP64 residual."""
+    boxes = [((8, 8, 40), (8.0, 80.0, 40.0)), ((24, 24, 24), (1.0,) * 3), ((3, 3, 3), (1.0,) * 3),
+             ((40, 9, 9), (40.0, 9.0, 90.0)), ((16, 20, 18), (1.0,) * 3),
+             ((48, 40, 36), (48.0, 40.0, 360.0))]
+    ss = [S.build(S.params(n=n, lengths=ln, seed=30 + i, dirichlet=S.FACE_XMIN))
+          for i, (n, ln) in enumerate(boxes)]
+    g = sv.GpuBatch([(s.neq, s.ia, s.ja) for s in ss], sv.CSRD, True)
+    g.set_values([s.al for s in ss], [s.ad for s in ss])
+    xs, infos = g.solve(sv.PCG, [s.b[0] for s in ss], tol=TOL, precision=precision)
+    for s, x, info in zip(ss, xs, infos):
+        args = (O.CSRD, True, s.ia, s.ja, s.al, s.ad)
+        assert info.status == sv.OK
+        if precision == sv.FP64:
+            ref = O.pcg(*args, s.b[0], tol=TOL)
+            d_it, d_x = O.order_spread(O.PCG, *args, s.b[0], tol=TOL)
+            assert abs(info.iters - ref.iters) <= max(1, 2 * d_it)
+            assert rel(x, ref.x) < max(BAR, 20 * d_x)
+        else:
+            r = s.b[0] - O.matvec(*args, x)
+            assert np.sqrt(abs(r @ (r / s.ad))) < TOL * np.sqrt(s.b[0] @ (s.b[0] / s.ad))
+            assert info.refinements >= 1
+    again, infos2 = g.solve(sv.PCG, [s.b[0] for s in ss], tol=TOL, precision=precision)
+    assert all(bits_equal(a, b) for a, b in zip(xs, again))
+    # the cap is each system's own, also past the first round
+    cap = max(i.iters for i in infos) - 5
+    _, capped = g.solve(sv.PCG, [s.b[0] for s in ss], tol=TOL, maxit=cap, precision=precision,
+                        raise_on_error=False)
+    assert [i.status for i in capped] == [sv.OK if i.iters <= cap else sv.MAXIT for i in infos]
+    g.close()
