@@ -2,8 +2,10 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "internal.h"
+#include "persist.cuh"
 
 namespace sfr {
 
@@ -59,7 +61,42 @@ __global__ void compensation_kernel(const int *sptr, const double *val, int n, i
   }
 }
 
+// Result records in pinned, device-mapped host memory: the kernel writes its
+// record there, so a solve needs no copy back.  One page per process, handed
+// out a record a call; a call that finds none free uses a device record.
+struct PinnedPool {
+  static constexpr int kRecords = 64;
+  std::mutex mu;
+  SolveOut *base = nullptr;
+  uint64_t used = 0;
+  bool tried = false;
+  SolveOut *take() {
+    std::lock_guard<std::mutex> lk(mu);
+    if (!tried) {
+      tried = true;
+      void *p = nullptr;
+      if (cudaHostAlloc(&p, sizeof(SolveOut) * kRecords,
+                        cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess)
+        base = static_cast<SolveOut *>(p);
+    }
+    if (!base || used == ~0ull) return nullptr;
+    const int i = __builtin_ctzll(~used);
+    used |= 1ull << i;
+    return base + i;
+  }
+  void give(SolveOut *r) {
+    std::lock_guard<std::mutex> lk(mu);
+    used &= ~(1ull << (r - base));
+  }
+};
+PinnedPool g_pool;
+
 }  // namespace
+
+ResultRecord::ResultRecord() : r(g_pool.take()) {}
+ResultRecord::~ResultRecord() {
+  if (r) g_pool.give(r);
+}
 
 int row_compensation(sfr_system *s, const DevSell &d, cudaStream_t st) {
   if (!s->d_comp) {

@@ -124,6 +124,15 @@ cudaError_t convert_diag32(const double *src, float *dst, int n, cudaStream_t st
 // d_comp from the FP64 and FP32 values of d (allocates d_comp on first use)
 int row_compensation(sfr_system *s, const DevSell &d, cudaStream_t st);
 
+// A call's result record in pinned, device-mapped host memory (null when none
+// is free): the kernel writes it there, so a solve needs no copy back.
+struct ResultRecord {
+  SolveOut *r;
+  ResultRecord();
+  ~ResultRecord();
+  ResultRecord(const ResultRecord &) = delete;
+};
+
 // kernels / solvers (krylov.cu)
 int solve_device(sfr_system *s, int32_t solver, int32_t k, const double *d_diag_k,
                  const double *d_b, double *d_x, double tol, uint32_t maxit,
@@ -149,15 +158,16 @@ int enqueue_team_mixed(sfr_system *s, int32_t solver, const double *d_b, double 
 
 // Resident engine (resident.cu): mixed PCG, one right-hand side, the
 // system's own diagonal.  resident_fits: the pattern and size allow it;
-// solve_resident returns SFR_UNSUPPORTED when the diagonal is not positive.
+// solve_resident returns SFR_UNSUPPORTED when the diagonal is not positive;
+// rdelta is the fall of the residual that asks for a refresh.
 // Self-tests of the bounded device-side waits (sfr_gpu_wait_selftest):
 // kind 0 grid_sync, 1 the fused iteration's tagged exchange; the resident
 // engine's exchange.
 int wait_selftest_fused(int32_t kind, int32_t absent, uint32_t spin_limit, cudaStream_t st);
 int wait_selftest_resident(int32_t absent, uint32_t spin_limit, cudaStream_t st);
 bool resident_fits(sfr_system *s);
-int solve_resident(sfr_system *s, const double *d_b, double *d_x, double tol, uint32_t maxit,
-                   int32_t newx, cudaStream_t st, sfr_solve_info *info);
+int solve_resident(sfr_system *s, const double *d_b, double *d_x, double tol, double rdelta,
+                   uint32_t maxit, int32_t newx, cudaStream_t st, sfr_solve_info *info);
 
 // On-chip engine (onchip.cu): FP64 PCG, one right-hand side.  SFR_UNSUPPORTED
 // when the system fits neither of its forms.

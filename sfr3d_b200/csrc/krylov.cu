@@ -616,6 +616,12 @@ namespace {
 
 // automatic engine choice: the graph engine from this many rows up
 constexpr int kGraphEngineRows = 100000;
+// mixed PCG: the resident engine from this many rows up.  An iteration of an
+// 8^3 box takes 2.0 us there and 8.9 us in the persistent kernel, of a 16^3 box
+// 3.6 and 7.8, of a 40^3 box 5.5 and 9.3, of a 56^3 box 6.6 and 14.  Below, a
+// solve is a few dozen iterations and may end exactly, where the norm that the
+// resident engine predicts for the next residual has no digits left.
+constexpr int kResidentRows = 512;
 
 struct Scratch {  // per-device scratch for the standalone reductions
   double *part = nullptr;
@@ -865,7 +871,7 @@ int enqueue_team_fp64(sfr_system *s, int32_t solver, const double *d_b, double *
 
 int auto_engine(sfr_system *s, int32_t solver, int32_t k, int32_t precision, bool own_diag) {
   const bool resident_case = precision == SFR_MIXED && solver == SFR_PCG && k == 1 && own_diag;
-  if (resident_case && s->n >= kGraphEngineRows && resident_fits(s)) return 4;
+  if (resident_case && s->n >= kResidentRows && resident_fits(s)) return 4;
   if (precision == SFR_FP64 && solver == SFR_PCG && k == 1 && s->graph_fused == kFusedOnChip)
     return 2;  // the on-chip engine, at every size
   return s->n >= kGraphEngineRows ? 2 : 1;
@@ -895,9 +901,17 @@ int solve_device(sfr_system *s, int32_t solver, int32_t k, const double *d_diag_
       tuned = true;
     }
   }
-  if (engine == 4 || (engine == 0 && resident_case && s->n >= kGraphEngineRows && resident_fits(s))) {
+  // the resident engine takes no call without iterations; the persistent one,
+  // which has the smaller systems otherwise, does
+  const bool resident_auto = resident_case && resident_fits(s) &&
+                             s->n >= (maxit ? kResidentRows : kGraphEngineRows);
+  if (engine == 4 || (engine == 0 && resident_auto)) {
     if (!resident_case) return SFR_UNSUPPORTED;
-    const int rc = solve_resident(s, d_b, d_x, tol, maxit, newx, st, info);
+    // a refresh costs a small system little, and keeps the FP32 recurrence of a
+    // badly conditioned one on course: there as often as in the persistent kernel
+    const double rdelta = engine == 0 && s->n < kGraphEngineRows ? reliable_delta(solver)
+                                                                 : reliable_delta_resident();
+    const int rc = solve_resident(s, d_b, d_x, tol, rdelta, maxit, newx, st, info);
     // automatic choice: a diagonal that is not positive has no Jacobi scaling
     if (rc != SFR_UNSUPPORTED || (engine == 4 && !tuned)) return rc;
   }

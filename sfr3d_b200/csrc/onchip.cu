@@ -603,43 +603,6 @@ __global__ void __launch_bounds__(kClusterThreads, 1) pcg_cluster_kernel(const C
 
 // ---- host ------------------------------------------------------------------
 
-// Result records in pinned, device-mapped host memory: the kernel writes its
-// record there, so a solve needs no copy back.  One page per process, handed
-// out a record a call; a call that finds none free uses a device record.
-struct PinnedPool {
-  static constexpr int kRecords = 64;
-  std::mutex mu;
-  SolveOut *base = nullptr;
-  uint64_t used = 0;
-  bool tried = false;
-  SolveOut *take() {
-    std::lock_guard<std::mutex> lk(mu);
-    if (!tried) {
-      tried = true;
-      void *p = nullptr;
-      if (cudaHostAlloc(&p, sizeof(SolveOut) * kRecords,
-                        cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess)
-        base = static_cast<SolveOut *>(p);
-    }
-    if (!base || used == ~0ull) return nullptr;
-    const int i = __builtin_ctzll(~used);
-    used |= 1ull << i;
-    return base + i;
-  }
-  void give(SolveOut *r) {
-    std::lock_guard<std::mutex> lk(mu);
-    used &= ~(1ull << (r - base));
-  }
-};
-PinnedPool g_pool;
-
-struct Record {
-  SolveOut *r = g_pool.take();
-  ~Record() {
-    if (r) g_pool.give(r);
-  }
-};
-
 int smem_optin(int device) {
   int v = 0;
   if (cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
@@ -896,7 +859,7 @@ int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double 
   }
   if (!s->ev0 && cudaEventCreate(&s->ev0) != cudaSuccess) return SFR_CUDA_ERROR;
   if (!s->ev1 && cudaEventCreate(&s->ev1) != cudaSuccess) return SFR_CUDA_ERROR;
-  Record rec;
+  ResultRecord rec;
   a.out = rec.r ? rec.r : dev_out;
   // stays when a wait gave up and the kernel left without a result
   SolveOut out{};
