@@ -28,7 +28,7 @@ NVCC = os.path.join(CUDA_HOME, "bin", "nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 CUDA_SOURCES = ["krylov.cu", "mixed.cu", "stream_solve.cu", "batched.cu", "device_mem.cu", "halo.cu",
-                "noalloc.cu", "adjoint.cu", "resident.cu", "onchip.cu", "mixed_team.cu", "krylov_ext.cu",
+                "noalloc.cu", "adjoint.cu", "resident.cu", "onchip.cu", "onchip_bicg.cu", "mixed_team.cu", "krylov_ext.cu",
                 "assembly.cu", "minres_graph.cu", "bicgl2_graph.cu", "gmres_graph.cu",
                 "gradient.cu"]
 HOST_SOURCES = ["capi.cpp", "sell_build.cpp", "partition.cpp", "autotune.cpp"]

@@ -195,6 +195,8 @@ extern "C" int sfr_gpu_autotune(sfr_system *s, int32_t solver, int32_t k, const 
   if (precision == SFR_FP64 && solver == SFR_PCG && k == 1) {
     for (int mode : {1, 2, 3, 4, kFusedOnChip}) add({2, 256, 0, 0, mode});
   }
+  if (precision == SFR_FP64 && solver == SFR_PBICGSTAB && onchip_bicg_fits(s, k, own_diag))
+    add({2, 256, 0, 0, kFusedOnChip});
   add({1, 0, 0, 0, 0});
   if (precision == SFR_MIXED && solver == SFR_PCG && k == 1 && own_diag && resident_fits(s))
     add({4, 0, 0, 0, 0});

@@ -105,7 +105,8 @@ struct sfr_system {
   int32_t graph_spw = 0;         // SELL slices per warp; 0: one wave of resident blocks
   int32_t graph_pf = 0;          // SpMV-phase L2 prefetch distance (rounds); 0: off
   // FP64 PCG, one RHS: 0 three kernels an iteration, 1-4 the fused iteration's
-  // modes, kFusedOnChip the on-chip engine (mode 4 where it does not fit)
+  // modes, kFusedOnChip the on-chip engine (mode 4 where it does not fit), of
+  // FP64 BiCGSTAB too
   int32_t graph_fused = sfr::kFusedOnChip;
   int32_t graph_stage = 0;       // BiCGSTAB SpMV phases: slices staged in shared memory
   std::vector<sfr::Tuned> tuned; // autotuned choices, used when engine == 0
@@ -173,6 +174,13 @@ int solve_resident(sfr_system *s, const double *d_b, double *d_x, double tol, do
 // when the system fits neither of its forms.
 int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double *d_x, double tol,
                  uint32_t maxit, int32_t newx, cudaStream_t st, sfr_solve_info *info);
+
+// On-chip BiCGSTAB (onchip_bicg.cu): FP64, up to three right-hand sides.
+// SFR_UNSUPPORTED when it does not fit, with nothing touched.
+bool onchip_bicg_fits(const sfr_system *s, int32_t k, bool own_diag);
+int solve_onchip_bicg(sfr_system *s, int32_t k, const double *d_diag_k, const double *d_b,
+                      double *d_x, double tol, uint32_t maxit, int32_t newx, cudaStream_t st,
+                      sfr_solve_info *info);
 
 // BiCGSTAB(2), GMRES(15), MINRES (krylov_ext.cu): one right-hand side, FP64;
 // d_diag null means the system's own diagonal

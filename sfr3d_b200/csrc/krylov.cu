@@ -874,6 +874,9 @@ int auto_engine(sfr_system *s, int32_t solver, int32_t k, int32_t precision, boo
   if (resident_case && s->n >= kResidentRows && resident_fits(s)) return 4;
   if (precision == SFR_FP64 && solver == SFR_PCG && k == 1 && s->graph_fused == kFusedOnChip)
     return 2;  // the on-chip engine, at every size
+  if (precision == SFR_FP64 && solver == SFR_PBICGSTAB && s->graph_fused == kFusedOnChip &&
+      onchip_bicg_fits(s, k, own_diag))
+    return 2;
   return s->n >= kGraphEngineRows ? 2 : 1;
 }
 
@@ -918,6 +921,11 @@ int solve_device(sfr_system *s, int32_t solver, int32_t k, const double *d_diag_
   if ((engine == 0 || engine == 2) && precision == SFR_FP64 && solver == SFR_PCG && k == 1 &&
       fused == kFusedOnChip) {
     const int rc = solve_onchip(s, d_diag_k, d_b, d_x, tol, maxit, newx, st, info);
+    if (rc != SFR_UNSUPPORTED) return rc;
+  }
+  if ((engine == 0 || engine == 2) && precision == SFR_FP64 && solver == SFR_PBICGSTAB &&
+      fused == kFusedOnChip) {
+    const int rc = solve_onchip_bicg(s, k, d_diag_k, d_b, d_x, tol, maxit, newx, st, info);
     if (rc != SFR_UNSUPPORTED) return rc;
   }
   if (fused == kFusedOnChip) fused = 4;

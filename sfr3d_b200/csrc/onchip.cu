@@ -68,7 +68,7 @@ struct ChipArgs {
 // square root and the quotient they name are formed only near their
 // thresholds, so an ordinary iteration waits on one division's latency.
 struct Scalars {
-  double conv, conv2, nu_old = 0.0, alpha = 0.0, beta = 0.0;
+  double conv, conv2, bnorm = 0.0, nu_old = 0.0, alpha = 0.0, beta = 0.0;
   int status = SFR_OK;
   unsigned iters = 0;
   __device__ __forceinline__ explicit Scalars(double c)
@@ -116,6 +116,7 @@ __device__ __forceinline__ void put_result(SolveOut *out, const Scalars &sc,
   o.norm_r_m = sqrt(fabs(tot[2]));
   o.norm_r = sqrt(tot[3]);
   o.conv = sc.conv;
+  o.bnorm = sc.bnorm;
   o.inner_iters = static_cast<int>(sc.iters);
   o.team_ms = ms;
   *out = o;
@@ -149,7 +150,7 @@ constexpr int kGridThreads = 768;
 // Where a system of a batched launch stands between two rounds (z, x and p
 // are in a.z, a.x and a.p).
 struct ChipState {
-  double conv, nu_old;
+  double conv, bnorm, nu_old;
   unsigned j;
   unsigned long long t0;  // its first round's start (global_ns)
 };
@@ -275,6 +276,7 @@ __device__ __forceinline__ bool pcg_grid_body(const ChipArgs &a, const TeamPart 
       const double d = __ldcg(a.diag + r0 + lr), b = ld_vec(a.b + r0 + lr);
       const double z = xdiv(b, d);
       acc[0] += b * z;
+      acc[1] += b * b;
       const double x0 = a.newx ? 0.0 : ld_vec(a.x + r0 + lr);
       if (kLevel >= 2 || a.newx) vx[lr] = x0;
       if (kLevel == 3) sm_d[lr] = d;
@@ -283,6 +285,7 @@ __device__ __forceinline__ bool pcg_grid_body(const ChipArgs &a, const TeamPart 
     }
     if (!team_sum<4, true>(a.sync, t, epoch, acc, tot, red, bad)) return false;
     sc = Scalars(a.tol * sqrt(fabs(tot[0])));
+    sc.bnorm = sqrt(tot[1]);
     if (!a.newx) {
       matvec([&](int lr, double y, double, double d, double) {
         vz[lr] = xdiv(xsub(ld_vec(a.b + r0 + lr), y), d);
@@ -294,6 +297,7 @@ __device__ __forceinline__ bool pcg_grid_body(const ChipArgs &a, const TeamPart 
     }
   } else {
     sc = Scalars(__ldcg(&st->conv));
+    sc.bnorm = __ldcg(&st->bnorm);
     sc.nu_old = __ldcg(&st->nu_old);
     j = __ldcg(&st->j);
     for (int lr = threadIdx.x; lr < own; lr += blockDim.x) {
@@ -336,6 +340,7 @@ __device__ __forceinline__ bool pcg_grid_body(const ChipArgs &a, const TeamPart 
       }
       if (static_cast<int>(blockIdx.x) == t.b0 && threadIdx.x == 0) {
         st->conv = sc.conv;
+        st->bnorm = sc.bnorm;
         st->nu_old = sc.nu_old;
         st->j = j + 1;
         if (!resume) st->t0 = t.t0;
@@ -534,6 +539,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) pcg_cluster_kernel(const C
     const double d = __ldg(a.diag + r0 + lr), b = ld_vec(a.b + r0 + lr);
     const double m = xdiv(1.0, d), z = xmul(b, m);
     acc[0] += b * z;
+    acc[1] += b * b;
     const double x0 = a.newx ? 0.0 : ld_vec(a.x + r0 + lr);
     if (kVecs) {
       sm_x[lr] = x0;
@@ -548,6 +554,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) pcg_cluster_kernel(const C
   cluster_sync_all();  // ex is zero in every block before the first exchange
   cluster_sum4(ex, buf, acc, tot, red);
   Scalars sc(a.tol * sqrt(fabs(tot[0])));
+  sc.bnorm = sqrt(tot[1]);
   if (!a.newx) {
     matvec([&](int lr, double y, double, double) {
       sm_z[lr] = xmul(xsub(ld_vec(a.b + r0 + lr), y), sm_m[lr]);
@@ -903,7 +910,7 @@ int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double 
     info->conv = out.conv;
     info->seconds = ms * 1e-3;
     info->inner_iters = out.inner_iters;
-    info->relres = std::nan("");
+    info->relres = out.bnorm > 0 ? out.norm_r / out.bnorm : 0.0;
   }
   return out.status;
 }

@@ -240,36 +240,31 @@ __device__ __forceinline__ unsigned round_cap(const RoundTable &rt, const TeamPa
   return max(16u, static_cast<unsigned>(fminf(us / rt.model.us(t.count, t.b1 - t.b0), 1e9f)));
 }
 
-// NV values (1, 2 or 4) summed over a warp, a butterfly that halves the
-// values a lane carries before it halves the lanes (four values: six 64-bit
-// shuffles instead of twenty).  Lane l ends with the total of value
+// NV values (a power of two up to 16) summed over a warp, a butterfly that
+// halves the values a lane carries before it halves the lanes (four values:
+// six 64-bit shuffles instead of twenty).  Lane l ends with the total of value
 // l >> kSumShift<NV>, the same bits in all the lanes that hold it.
 template <int NV>
-constexpr int kSumShift = NV == 4 ? 3 : NV == 2 ? 4 : 5;
+constexpr int kSumShift = NV == 16 ? 1 : NV == 8 ? 2 : NV == 4 ? 3 : NV == 2 ? 4 : 5;
 
-template <int NV>
+template <int NV, int kLanes = 16>
 __device__ __forceinline__ double warp_sum_n(const double (&v)[NV]) {
-  static_assert(NV == 1 || NV == 2 || NV == 4, "one, two or four values");
-  const int lane = threadIdx.x & 31;
+  static_assert(NV == 1 || NV == 2 || NV == 4 || NV == 8 || NV == 16, "a power of two");
   constexpr unsigned kAll = 0xffffffffu;
-  double t;
-  if constexpr (NV == 4) {
-    const bool h16 = lane & 16, h8 = lane & 8;
-    const double a0 = (h16 ? v[2] : v[0]) + __shfl_xor_sync(kAll, h16 ? v[0] : v[2], 16);
-    const double a1 = (h16 ? v[3] : v[1]) + __shfl_xor_sync(kAll, h16 ? v[1] : v[3], 16);
-    t = (h8 ? a1 : a0) + __shfl_xor_sync(kAll, h8 ? a0 : a1, 8);
-  } else if constexpr (NV == 2) {
-    const bool h16 = lane & 16;
-    t = (h16 ? v[1] : v[0]) + __shfl_xor_sync(kAll, h16 ? v[0] : v[1], 16);
-    t += __shfl_xor_sync(kAll, t, 8);
+  if constexpr (NV == 1) {
+    double t = v[0];
+#pragma unroll
+    for (int o = kLanes; o > 0; o >>= 1) t += __shfl_xor_sync(kAll, t, o);
+    return t;
   } else {
-    t = v[0] + __shfl_xor_sync(kAll, v[0], 16);
-    t += __shfl_xor_sync(kAll, t, 8);
+    const bool hi = threadIdx.x & kLanes;
+    double h[NV / 2];
+#pragma unroll
+    for (int i = 0; i < NV / 2; ++i)
+      h[i] = (hi ? v[i + NV / 2] : v[i]) +
+             __shfl_xor_sync(kAll, hi ? v[i] : v[i + NV / 2], kLanes);
+    return warp_sum_n<NV / 2, kLanes / 2>(h);
   }
-  t += __shfl_xor_sync(kAll, t, 4);
-  t += __shfl_xor_sync(kAll, t, 2);
-  t += __shfl_xor_sync(kAll, t, 1);
-  return t;
 }
 
 // Whether this lane writes the total it holds.
