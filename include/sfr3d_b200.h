@@ -242,6 +242,22 @@ int sfr_gpu_adjoint(sfr_system *s, int32_t solver, const double *x,
                     double *g_au, double tol, uint32_t maxit,
                     int32_t precision, sfr_solve_info *info);
 
+/* sfr_gpu_set_values and sfr_gpu_adjoint with everything on the system's device.  d_src holds the
+ * nsrc stored values (al, for CSRC unsym al then au; another count is
+ * SFR_BAD_INPUT), d_gsrc their
+ * gradients in the same order; the other arrays are n doubles.  The inputs
+ * may still be in the making on `stream` (NULL: the legacy default stream);
+ * the outputs are complete on return.  d_lam, d_gsrc and d_gad overlap
+ * neither each other nor an input. */
+int sfr_gpu_set_values_device(sfr_system *s, int32_t nsrc,
+                              const double *d_src, const double *d_ad,
+                              void *stream);
+int sfr_gpu_adjoint_device(sfr_system *s, int32_t solver, int32_t nsrc,
+                           const double *d_x, const double *d_g,
+                           double *d_lam, double *d_gsrc, double *d_gad,
+                           double tol, uint32_t maxit, int32_t precision,
+                           void *stream, sfr_solve_info *info);
+
 int sfr_gpu_destroy(sfr_system *s);
 
 /* ---- batches of independent systems ----------------------------------- */

@@ -4,7 +4,8 @@ For a scalar J(x) with g = dJ/dx the adjoint system is A^T lam = g; then
 dJ/db = lam and dJ/dA_ij = -lam_i x_j for every (i, j) of the stored
 pattern.  The GPU work (transpose solve on the transposed SELL copy, the
 gradient scatter into the caller's value layout) is one C-ABI call,
-``sfr_gpu_adjoint``; this module only adapts it to torch tensors.
+``sfr_gpu_adjoint``; this module only adapts it to torch tensors (tensors on
+the system's GPU stay there: ``sfr_gpu_adjoint_device``).
 
 The reference solves forward systems only (Solv.c:64-501, Bicgstab.c:57);
 the transpose solve reuses its BiCGSTAB iteration on A^T.  A value that the
@@ -42,6 +43,37 @@ def _np(t):
 
 if torch is not None:
 
+    def _on_device(system, al, ad, au, b):
+        """The stored values [al | au], ad and b as private FP64 copies on the
+        system's GPU, or None for the host path: tensors elsewhere, counts
+        that are not the pattern's (the host entries do not look at them), a
+        stream that is being captured.
+
+        Forward and backward of a 48^3 system take 0.59 ms so; through host
+        memory 4.76, of which the two solves are 0.16 (30 MB through pageable
+        memory, and a device allocation)."""
+        split = system.storage == CSRC and system.unsym
+        src = [al, au] if split and au is not None else [al]
+        plain = (torch.Tensor, torch.nn.Parameter)
+        given = [t for t in (al, ad, au, b) if t is not None]
+        if not all(type(t) in plain and t.layout == torch.strided and t.is_cuda
+                   and t.get_device() == system.device and not t.is_complex() for t in given):
+            return None
+        n, nsrc = system.neq, system._nsrc()
+        if sum(t.numel() for t in src) != nsrc or (len(src) == 2 and al.numel() != au.numel()):
+            return None
+        if ad.numel() != n or b.numel() != n:
+            return None
+        with torch.cuda.device(system.device):
+            if torch.cuda.is_current_stream_capturing():
+                return None
+        return (torch.cat([t.detach().reshape(-1).to(torch.float64) for t in src]),
+                ad.detach().reshape(-1).to(torch.float64, copy=True),
+                b.detach().reshape(-1).to(torch.float64, copy=True))
+
+    def _stream(system):
+        return torch.cuda.current_stream(system.device).cuda_stream
+
     class LinearSolve(torch.autograd.Function):
         """x = A(al, ad, au)^-1 b on the pattern of a GpuSystem.
 
@@ -49,21 +81,38 @@ if torch is not None:
         value arrays of ``GpuSystem.set_values`` (au may be None), b the
         right-hand side; opts = (tol, maxit, precision) of the forward and
         the adjoint solve.  Forward and backward go through the C ABI;
-        tensors are staged through host memory.
+        tensors that are not on the system's GPU are staged through host
+        memory.
         """
 
         @staticmethod
         def forward(ctx, system, solver, opts, al, ad, au, b):
             tol, maxit, precision = opts
+            ctx.system, ctx.solver, ctx.opts = system, solver, opts
+            ctx.has_au = au is not None
+            dev = _on_device(system, al, ad, au, b)
+            ctx.device = dev is not None
+            if dev is not None:
+                src, diag, rhs = dev
+                x = torch.empty_like(rhs)
+                system.set_values_device(src.numel(), src.data_ptr(), diag.data_ptr(),
+                                         _stream(system))
+                # no work touches rhs and x but what set_values_device waited for
+                info = system.solve_device(solver, rhs.data_ptr(), x.data_ptr(), tol=tol,
+                                           maxit=maxit, precision=precision)
+                if info.status != 0:
+                    raise SolverError(info.status, "LinearSolve.forward")
+                ctx.values = (src, diag)
+                ctx.version = system.values_version
+                ctx.x = x.clone()  # the caller may write to x
+                return x
             system.set_values(_np(al), _np(ad), _np(au))
             x, info = system.solve(solver, _np(b), tol=tol, maxit=maxit,
                                    precision=precision)
             if info.status != 0:
                 raise SolverError(info.status, "LinearSolve.forward")
-            ctx.system, ctx.solver, ctx.opts = system, solver, opts
             ctx.values = (_np(al), _np(ad), _np(au))
             ctx.version = system.values_version
-            ctx.has_au = au is not None
             ctx.x = x
             return torch.from_numpy(x).to(b.device)
 
@@ -71,6 +120,8 @@ if torch is not None:
         def backward(ctx, gx):
             system = ctx.system
             tol, maxit, precision = ctx.opts
+            if ctx.device:
+                return LinearSolve._backward_device(ctx, gx)
             if system.values_version != ctx.version:
                 system.set_values(*ctx.values)
                 ctx.version = system.values_version
@@ -83,6 +134,29 @@ if torch is not None:
             t = lambda a: None if a is None else torch.from_numpy(a).to(dev)
             return (None, None, None, t(g_al), t(g_ad),
                     t(g_au) if ctx.has_au else None, t(lam))
+
+        @staticmethod
+        def _backward_device(ctx, gx):
+            system = ctx.system
+            tol, maxit, precision = ctx.opts
+            src, diag = ctx.values
+            if system.values_version != ctx.version:
+                system.set_values_device(src.numel(), src.data_ptr(), diag.data_ptr(),
+                                         _stream(system))
+                ctx.version = system.values_version
+            g = gx.detach().resolve_neg().to(torch.float64).contiguous()
+            g_src = torch.empty_like(src)
+            g_ad, lam = torch.empty_like(diag), torch.empty_like(diag)
+            info = system.adjoint_device(
+                ctx.solver, src.numel(), ctx.x.data_ptr(), g.data_ptr(), lam.data_ptr(),
+                g_src.data_ptr(), g_ad.data_ptr(), tol=tol, maxit=maxit, precision=precision,
+                stream=_stream(system))
+            if info.status != 0:
+                raise SolverError(info.status, "LinearSolve.backward")
+            split = system.storage == CSRC and system.unsym
+            half = src.numel() // 2 if split else src.numel()
+            return (None, None, None, g_src[:half], g_ad,
+                    g_src[half:] if ctx.has_au and split else None, lam)
 
     def linear_solve(system: GpuSystem, al, ad, b, au=None,
                      solver: int = PBICGSTAB, tol: float = 1e-12,

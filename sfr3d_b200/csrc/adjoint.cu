@@ -40,11 +40,32 @@ __global__ void grad_diag_kernel(const double *lam, const double *x, int n, doub
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) g_ad[i] = -(lam[i] * x[i]);
 }
 
+__global__ void any_nonzero_kernel(const double *g, int n, int *flag) {
+  const int stride = gridDim.x * blockDim.x;
+  bool any = false;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) any |= !(g[i] == 0.0);
+  if (any) *flag = 1;
+}
+
 }  // namespace
+
+int any_nonzero(const double *d_g, int n, int *d_flag, int *flag, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(d_flag, 0, sizeof(int), st);
+  if (e == cudaSuccess) {
+    any_nonzero_kernel<<<std::max(1, std::min((n + 255) / 256, 1184)), 256, 0, st>>>(d_g, n,
+                                                                                    d_flag);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) return SFR_OK;
+  set_last_error(cudaGetErrorString(e));
+  return SFR_CUDA_ERROR;
+}
 
 int adjoint_gradients(sfr_system *s, const double *d_lam, const double *d_x, double *d_gsrc,
                       double *d_gad, cudaStream_t st) {
-  if (cudaMemsetAsync(d_gsrc, 0, sizeof(double) * std::max(s->nsrc, 1), st) != cudaSuccess)
+  if (s->nsrc > 0 && cudaMemsetAsync(d_gsrc, 0, sizeof(double) * s->nsrc, st) != cudaSuccess)
     return SFR_CUDA_ERROR;
   const int grid = static_cast<int>(
       std::min<int64_t>((static_cast<int64_t>(s->A.nslices) * 32 + 255) / 256, 4096));

@@ -209,6 +209,36 @@ int sfr_gpu_set_values(sfr_system *s, const double *al, const double *ad, const 
   return SFR_OK;
 }
 
+namespace {
+
+// The device entries take inputs that the caller's stream may still be
+// writing: `st` goes on after what is in that stream now.
+int follow(sfr_system *s, cudaStream_t caller, cudaStream_t st) {
+  if (!s->ev0) SFR_CU(cudaEventCreate(&s->ev0));
+  SFR_CU(cudaEventRecord(s->ev0, caller));
+  SFR_CU(cudaStreamWaitEvent(st, s->ev0, 0));
+  return SFR_OK;
+}
+
+}  // namespace
+
+int sfr_gpu_set_values_device(sfr_system *s, int32_t nsrc, const double *d_src,
+                              const double *d_ad, void *stream) {
+  if (!s || nsrc != s->nsrc || !d_ad || (!d_src && nsrc > 0)) return SFR_BAD_INPUT;
+  SFR_CU(cudaSetDevice(s->device));
+  int rc = follow(s, static_cast<cudaStream_t>(stream), s->stream);
+  if (rc != SFR_OK) return rc;
+  if (s->nsrc > 0)
+    SFR_CU(cudaMemcpyAsync(s->d_stage, d_src, sizeof(double) * s->nsrc, cudaMemcpyDeviceToDevice,
+                           s->stream));
+  SFR_CU(cudaMemcpyAsync(s->d_diag, d_ad, sizeof(double) * s->n, cudaMemcpyDeviceToDevice,
+                         s->stream));
+  rc = sfr::values_refreshed(s, s->stream);
+  if (rc != SFR_OK) return rc;
+  SFR_CU(cudaStreamSynchronize(s->stream));
+  return SFR_OK;
+}
+
 // Matrix Market dumps as the reference writes them (WriteMtx.c:26-179 with
 // its vendored writer): the diagonal then the stored entries of each row,
 // 1-based, "%d %d %30.14e"; values al below the diagonal and, for unsym, au
@@ -547,6 +577,44 @@ int sfr_gpu_adjoint(sfr_system *s, int32_t solver, const double *x, const double
   }
   cudaFree(d_gad);
   return rc;
+}
+
+int sfr_gpu_adjoint_device(sfr_system *s, int32_t solver, int32_t nsrc, const double *d_x,
+                           const double *d_g, double *d_lam, double *d_gsrc, double *d_gad,
+                           double tol, uint32_t maxit, int32_t precision, void *stream,
+                           sfr_solve_info *info) {
+  if (!s || nsrc != s->nsrc || !d_x || !d_g || !d_lam || !d_gad || (!d_gsrc && nsrc > 0))
+    return SFR_BAD_INPUT;
+  if (!s->values_set) return SFR_BAD_INPUT;
+  SFR_CU(cudaSetDevice(s->device));
+  sfr_system *t = nullptr;
+  int rc = transpose_view(s, &t);
+  if (rc != SFR_OK) return rc;
+  rc = follow(s, static_cast<cudaStream_t>(stream), t->stream);
+  if (rc != SFR_OK) return rc;
+  // s->ev0 is behind the caller's stream, so after the wait for this flag
+  // everything the gradients read is ready on any stream
+  IoBuffers *io = nullptr;
+  rc = io_for(s, 1, &io);
+  if (rc != SFR_OK) return rc;
+  int nonzero = 0;
+  rc = sfr::any_nonzero(d_g, s->n, reinterpret_cast<int *>(io->diag), &nonzero, t->stream);
+  if (rc != SFR_OK) return rc;
+  if (!nonzero) {  // as in sfr_gpu_adjoint
+    SFR_CU(cudaMemsetAsync(d_lam, 0, sizeof(double) * s->n, t->stream));
+    if (s->nsrc > 0) SFR_CU(cudaMemsetAsync(d_gsrc, 0, sizeof(double) * s->nsrc, t->stream));
+    SFR_CU(cudaMemsetAsync(d_gad, 0, sizeof(double) * s->n, t->stream));
+    SFR_CU(cudaStreamSynchronize(t->stream));
+    if (info) *info = sfr_solve_info{};
+    return SFR_OK;
+  }
+  rc = sfr::solve_device(t, solver, 1, nullptr, d_g, d_lam, tol, maxit, 1, precision, t->stream,
+                         info);
+  if (rc != SFR_OK) return rc;
+  rc = sfr::adjoint_gradients(s, d_lam, d_x, d_gsrc, d_gad, t->stream);
+  if (rc != SFR_OK) return rc;
+  SFR_CU(cudaStreamSynchronize(t->stream));
+  return SFR_OK;
 }
 
 int sfr_gpu_spmv(sfr_system *s, const double *d_x, double *d_y, void *stream) {

@@ -228,7 +228,10 @@ int auto_engine(sfr_system *s, int32_t solver, int32_t k, int32_t precision, boo
 // Blocks of the standalone dot / SpMV+dot kernels (256 threads each) for n
 // elements on `device`: 4 per SM of the device, at most one per 256 elements.
 int stat_grid(int device, int64_t n);
-// adjoint.cu: dJ/d(value source) and dJ/d(ad) from lam and x (device arrays)
+// adjoint.cu: whether any of n values is not zero (a NaN is not; d_flag: 4
+// bytes of scratch; waits for `st`)
+int any_nonzero(const double *d_g, int n, int *d_flag, int *flag, cudaStream_t st);
+// dJ/d(value source) and dJ/d(ad) from lam and x (device arrays)
 int adjoint_gradients(sfr_system *s, const double *d_lam, const double *d_x, double *d_gsrc,
                       double *d_gad, cudaStream_t st);
 // Text for sfr_last_error() (capi.cpp)

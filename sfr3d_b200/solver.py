@@ -105,6 +105,9 @@ def lib() -> ctypes.CDLL:
                                           ctypes.c_uint32, _I32, _I32, _P]
     L.sfr_gpu_adjoint.argtypes = [_P, _I32, _P, _P, _P, _P, _P, _P,
                                   ctypes.c_double, ctypes.c_uint32, _I32, _P]
+    L.sfr_gpu_set_values_device.argtypes = [_P, _I32, _P, _P, _P]
+    L.sfr_gpu_adjoint_device.argtypes = [_P, _I32, _I32, _P, _P, _P, _P, _P, ctypes.c_double,
+                                         ctypes.c_uint32, _I32, _P, _P]
     L.sfr_gpu_destroy.argtypes = [_P]
     L.sfr_gpu_set_engine.argtypes = [_P, _I32, _I32, _I32]
     L.sfr_gpu_set_prefetch.argtypes = [_P, _I32]
@@ -208,6 +211,7 @@ class GpuSystem:
         if rc != OK:
             raise SolverError(rc, "sfr_gpu_create")
         self.h = h
+        self.device = device
 
     def close(self):
         if getattr(self, "h", None):
@@ -397,6 +401,26 @@ class GpuSystem:
         if rc < 0:
             raise SolverError(rc, "sfr_gpu_solve_multi_device")
         return [SolveInfo.from_c(infos[i]) for i in range(k)]
+
+    def set_values_device(self, nsrc: int, d_src: int, d_ad: int, stream: int = 0):
+        """set_values from device arrays that work on `stream` may still be
+        writing: the nsrc stored values (al, for CSRC unsym al then au) and
+        the diagonal."""
+        rc = lib().sfr_gpu_set_values_device(self.h, nsrc, d_src or None, d_ad, stream or None)
+        if rc != OK:
+            raise SolverError(rc, "sfr_gpu_set_values_device: " + last_error())
+        self.values_version += 1
+
+    def adjoint_device(self, solver, nsrc: int, d_x: int, d_g: int, d_lam: int, d_gsrc: int,
+                       d_gad: int, tol=1e-12, maxit=100000, precision=FP64, stream: int = 0):
+        """adjoint on device arrays (sfr_gpu_adjoint_device)."""
+        info = SolveInfoC()
+        rc = lib().sfr_gpu_adjoint_device(self.h, solver, nsrc, d_x, d_g, d_lam, d_gsrc or None,
+                                          d_gad, tol, maxit, precision, stream or None,
+                                          ctypes.byref(info))
+        if rc < 0:
+            raise SolverError(rc, "sfr_gpu_adjoint_device: " + last_error())
+        return SolveInfo.from_c(info)
 
     def spmv(self, d_x: int, d_y: int, stream: int = 0):
         rc = lib().sfr_gpu_spmv(self.h, d_x, d_y, stream or None)
