@@ -56,7 +56,11 @@ extern "C" {
 
 /* precision modes */
 #define SFR_FP64 0           /* plain FP64: the reference's arithmetic */
-#define SFR_MIXED 1          /* FP32 matrix + inner Krylov, FP64 refinement */
+/* FP32 matrix + inner Krylov, FP64 refinement.  BiCGSTAB on up to three
+ * right-hand sides of a system that the on-chip engine holds runs there in
+ * FP64 throughout, which is faster (refinements 0), unless an engine was
+ * chosen (sfr_gpu_set_engine). */
+#define SFR_MIXED 1
 
 typedef struct sfr_system sfr_system; /* one pattern resident on a device */
 

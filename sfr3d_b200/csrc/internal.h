@@ -222,8 +222,9 @@ int num_sms(int device);
 // The autotuned choice for this kind of solve, or null (autotune.cpp).
 const Tuned *find_tuned(const sfr_system *s, int32_t solver, int32_t k, int32_t precision,
                         bool own_diag);
-// The automatic engine choice without a tuned entry: 1 persistent, 2 graph,
-// 4 resident (krylov.cu).
+// The automatic engine choice without a tuned entry: 1 persistent, 2 graph
+// (FP64: on-chip when it fits), 4 resident; 0 where no engine number names it
+// (mixed BiCGSTAB on chip) (krylov.cu).
 int auto_engine(sfr_system *s, int32_t solver, int32_t k, int32_t precision, bool own_diag);
 // Blocks of the standalone dot / SpMV+dot kernels (256 threads each) for n
 // elements on `device`: 4 per SM of the device, at most one per 256 elements.

@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 
 #include "common.cuh"
@@ -869,14 +870,37 @@ int enqueue_team_fp64(sfr_system *s, int32_t solver, const double *d_b, double *
              : SFR_CUDA_ERROR;
 }
 
+// BiCGSTAB solves that go to the on-chip engine when they fit it: FP64 under
+// the automatic choice and engine 2, and, under the automatic choice, mixed
+// ones too, in FP64 throughout.  On chip an iteration waits on exchanges and
+// gathers, not on bytes, so FP32 inner vectors would gain little, and the
+// reliable updates' FP64 passes fall away.  Mixed kernels against this one, us
+// a solve of one / three systems: 8^3 105 / 180 and 45 / 54, 40^3 226 / 401
+// and 94 / 109, 60^3 401 / 641 and 151 / 210, 76^3 513 / 984 and 210 / 521,
+// 92^3 of one 768 and 498.
+static bool onchip_bicg_case(const sfr_system *s, int32_t solver, int32_t precision, int32_t engine,
+                      int32_t fused) {
+  return solver == SFR_PBICGSTAB && fused == kFusedOnChip &&
+         ((precision == SFR_FP64 && (engine == 0 || engine == 2)) ||
+          (precision == SFR_MIXED && engine == 0));
+}
+
+// Whether k right-hand sides' x shares memory with b or their diagonals.
+static bool overlaps_input(int n, int k, const double *x, const double *b, const double *diag) {
+  const uintptr_t nb = sizeof(double) * static_cast<uintptr_t>(n) * k;
+  const auto at = [](const double *p) { return reinterpret_cast<uintptr_t>(p); };
+  const auto meets = [&](uintptr_t p) { return at(x) < p + nb && p < at(x) + nb; };
+  return meets(at(b)) || (diag && meets(at(diag)));
+}
+
 int auto_engine(sfr_system *s, int32_t solver, int32_t k, int32_t precision, bool own_diag) {
   const bool resident_case = precision == SFR_MIXED && solver == SFR_PCG && k == 1 && own_diag;
   if (resident_case && s->n >= kResidentRows && resident_fits(s)) return 4;
   if (precision == SFR_FP64 && solver == SFR_PCG && k == 1 && s->graph_fused == kFusedOnChip)
     return 2;  // the on-chip engine, at every size
-  if (precision == SFR_FP64 && solver == SFR_PBICGSTAB && s->graph_fused == kFusedOnChip &&
+  if (onchip_bicg_case(s, solver, precision, 0, s->graph_fused) &&
       onchip_bicg_fits(s, k, own_diag))
-    return 2;
+    return precision == SFR_FP64 ? 2 : 0;
   return s->n >= kGraphEngineRows ? 2 : 1;
 }
 
@@ -923,18 +947,37 @@ int solve_device(sfr_system *s, int32_t solver, int32_t k, const double *d_diag_
     const int rc = solve_onchip(s, d_diag_k, d_b, d_x, tol, maxit, newx, st, info);
     if (rc != SFR_UNSUPPORTED) return rc;
   }
-  if ((engine == 0 || engine == 2) && precision == SFR_FP64 && solver == SFR_PBICGSTAB &&
-      fused == kFusedOnChip) {
-    const int rc = solve_onchip_bicg(s, k, d_diag_k, d_b, d_x, tol, maxit, newx, st, info);
-    if (rc != SFR_UNSUPPORTED) return rc;
+  int32_t iters0[kMaxK] = {};  // iterations before the engine below
+  if (onchip_bicg_case(s, solver, precision, engine, fused)) {
+    sfr_solve_info mine[kMaxK];
+    const int rc = solve_onchip_bicg(s, k, d_diag_k, d_b, d_x, tol, maxit, newx, st, mine);
+    if (rc != SFR_UNSUPPORTED) {
+      // a mixed solve ends on the true residual: where the recurrence's has
+      // left it behind (tolerances near FP64's floor), the mixed engine goes on,
+      // if x was not written over what it reads
+      bool met = true;
+      if (rc == SFR_OK && precision == SFR_MIXED && !overlaps_input(s->n, k, d_x, d_b, d_diag_k))
+        for (int i = 0; i < k; ++i) met = met && mine[i].norm_r < mine[i].conv;
+      if (met) {
+        if (info && rc >= 0) std::copy(mine, mine + k, info);
+        return rc;
+      }
+      newx = 0;
+      for (int i = 0; i < k; ++i) iters0[i] = mine[i].iters;
+    }
   }
   if (fused == kFusedOnChip) fused = 4;
   if (engine == 0 || engine == 4) engine = s->n >= kGraphEngineRows ? 2 : 1;
+  const auto total = [&](int rc) {
+    for (int i = 0; i < k && info && rc >= 0; ++i) info[i].iters += iters0[i];
+    return rc;
+  };
   if (engine == 2 || engine == 3)
-    return solve_stream(s, solver, k, d_diag_k, d_b, d_x, tol, maxit, newx, precision,
-                        reliable_delta(solver), threads, spw, pf, fused, engine == 3, st, info);
+    return total(solve_stream(s, solver, k, d_diag_k, d_b, d_x, tol, maxit, newx, precision,
+                              reliable_delta(solver), threads, spw, pf, fused, engine == 3, st,
+                              info));
   if (precision == SFR_MIXED)
-    return solve_mixed(s, solver, k, d_diag_k, d_b, d_x, tol, maxit, newx, st, info);
+    return total(solve_mixed(s, solver, k, d_diag_k, d_b, d_x, tol, maxit, newx, st, info));
   if (precision != SFR_FP64) return SFR_UNSUPPORTED;
   SolveOut out[kMaxK];
   float ms = 0.f;
