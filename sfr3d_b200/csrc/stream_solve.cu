@@ -98,6 +98,7 @@ struct SState {
   SCall call;
   double d[K], alpha[K], beta[K], omega[K], rr0[K], conv[K], bnorm[K], rmax[K];
   int active[K], iters[K], status[K], refine[K], upd[K];
+  int pend[K];  // BiCGSTAB: what x still lacks of this iteration (kPendAlpha | kPendOmega)
   int any, any_upd;
   unsigned j;
   SolveOut out[K];
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(256) k_setup(const SArgs<K> a, SState<K> *st) 
       st->status[k] = SFR_OK;
       st->refine[k] = 0;
       st->upd[k] = 0;
+      st->pend[k] = 0;
       st->beta[k] = 0.0;
     }
     st->j = 0;
@@ -910,6 +912,14 @@ __global__ void __launch_bounds__(256) k_post(const SArgs<K> a, SState<K> *st) {
 // =========================== BiCGSTAB ====================================
 // FP64: Bicgstab.c:50-245.  Vectors: r0 shadow, p (p0), z = M p or M s,
 // v (q), t.  Mixed: the same in FP32 with xs and reliable updates.
+//
+// x += alpha M p + w z is left to phase C, which holds M and p anyway, and has
+// z before it overwrites it: M p has the bits of the z that phase A1 gathered.
+// B1 and B2 are bound by memory; without x and z they move 8 vectors a
+// right-hand side and iteration instead of 14, C 8 instead of 5 (three right-hand
+// sides: mixed 128^3 4.47 -> 4.34 ms, FP64 110x99x105 2.52 -> 2.43).  st->pend says which of the two terms of
+// the running iteration x lacks, of a system that stopped in it too.
+constexpr int kPendAlpha = 1, kPendOmega = 2;
 
 template <int K, bool kMixed, typename I>
 __global__ void __launch_bounds__(256) k_bicg_start(const SArgs<K> a, SState<K> *st) {
@@ -963,6 +973,7 @@ __global__ void __launch_bounds__(256) k_bicg_start(const SArgs<K> a, SState<K> 
 template <int K, bool kMixed, typename I, int kStages = 0>
 __global__ void __launch_bounds__(256, (SpmvShape<K, kMixed>::kMinBlocks)) k_bicg_a1(const SArgs<K> a, SState<K> *st) {
   SFR_SHARED_RED(2 * K);
+  if (blockIdx.x == 0 && threadIdx.x < K) st->pend[threadIdx.x] = 0;
   if (!st->any) return;
   const int n = a.n;
   const int lane = threadIdx.x & 31;
@@ -1045,7 +1056,7 @@ __global__ void __launch_bounds__(256, (SpmvShape<K, kMixed>::kMinBlocks)) k_bic
   }
 }
 
-// B1: x += alpha z ; s = r -= alpha v ; z = M s ; (s, s) ; half-step test
+// B1: s = r -= alpha v ; z = M s ; (s, s) ; half-step test
 template <int K, bool kMixed>
 __global__ void __launch_bounds__(256) k_bicg_b1(const SArgs<K> a, SState<K> *st) {
   SFR_SHARED_RED(K);
@@ -1067,26 +1078,20 @@ __global__ void __launch_bounds__(256) k_bicg_b1(const SArgs<K> a, SState<K> *st
       if (!act[k]) continue;
       if (!kMixed) {
         const double al = alv[k];
-        const double2 zv = ld2(a.z[k] + r), q = ld2ro(a.q[k] + r), m = ld2ro(a.m[k] + r);
-        double2 xv = ld2(a.x[k] + r), rv = ld2(a.r[k] + r);
-        xv.x = xadd(xv.x, xmul(al, zv.x));
-        xv.y = xadd(xv.y, xmul(al, zv.y));
+        const double2 q = ld2ro(a.q[k] + r), m = ld2ro(a.m[k] + r);
+        double2 rv = ld2(a.r[k] + r);
         rv.x = xsub(rv.x, xmul(al, q.x));
         rv.y = xsub(rv.y, xmul(al, q.y));
-        st2(a.x[k] + r, xv);
         st2(a.r[k] + r, rv);
         st2(a.z[k] + r, make_double2(xmul(rv.x, m.x), xmul(rv.y, m.y)));
         acc[k] += rv.x * rv.x;
         if (two) acc[k] += rv.y * rv.y;
       } else {
         const float af = static_cast<float>(alv[k]);
-        const float2 zv = ld2(a.fz[k] + r), q = ld2ro(a.fq[k] + r), m = ld2ro(a.m32[k] + r);
-        float2 xs = ld2(a.fxs[k] + r), rv = ld2(a.fr[k] + r);
-        xs.x = fmaf(af, zv.x, xs.x);
-        xs.y = fmaf(af, zv.y, xs.y);
+        const float2 q = ld2ro(a.fq[k] + r), m = ld2ro(a.m32[k] + r);
+        float2 rv = ld2(a.fr[k] + r);
         rv.x = fmaf(-af, q.x, rv.x);
         rv.y = fmaf(-af, q.y, rv.y);
-        st2(a.fxs[k] + r, xs);
         st2(a.fr[k] + r, rv);
         st2(a.fz[k] + r, make_float2(m.x * rv.x, m.y * rv.y));
         acc[k] += static_cast<double>(rv.x) * static_cast<double>(rv.x);
@@ -1101,6 +1106,7 @@ __global__ void __launch_bounds__(256) k_bicg_b1(const SArgs<K> a, SState<K> *st
     for (int k = 0; k < K; ++k) {
       st->upd[k] = 0;
       if (!act[k]) continue;
+      st->pend[k] = kPendAlpha;
       if (sqrt(sm[k]) < st->conv[k]) {
         if (kMixed) {
           st->upd[k] = 1;  // confirm on the FP64 true residual
@@ -1162,6 +1168,7 @@ __global__ void __launch_bounds__(256) k_bicg_refresh(const SArgs<K> a, SState<K
       if (sel[k]) {
         st->refine[k] += 1;
         st->upd[k] = 0;
+        st->pend[k] = 0;  // k_bicg_fold added it
         const double tr = sqrt(sm[2 * k]);
         if (tr < st->conv[k]) {
           st->active[k] = 0;
@@ -1262,7 +1269,7 @@ __global__ void __launch_bounds__(256, (SpmvShape<K, kMixed>::kMinBlocks)) k_bic
   }
 }
 
-// B2: x += w z ; r -= w t ; (r, r), (r, r0) ; full-step test, beta
+// B2: r -= w t ; (r, r), (r, r0) ; full-step test, beta
 template <int K, bool kMixed>
 __global__ void __launch_bounds__(256) k_bicg_b2(const SArgs<K> a, SState<K> *st) {
   SFR_SHARED_RED(2 * K);
@@ -1283,13 +1290,10 @@ __global__ void __launch_bounds__(256) k_bicg_b2(const SArgs<K> a, SState<K> *st
       if (!act[k]) continue;
       if (!kMixed) {
         const double w = omv[k];
-        const double2 zv = ld2ro(a.z[k] + r), tv = ld2ro(a.t[k] + r), r0 = ld2ro(a.r0[k] + r);
-        double2 xv = ld2(a.x[k] + r), rv = ld2(a.r[k] + r);
-        xv.x = xadd(xv.x, xmul(w, zv.x));
-        xv.y = xadd(xv.y, xmul(w, zv.y));
+        const double2 tv = ld2ro(a.t[k] + r), r0 = ld2ro(a.r0[k] + r);
+        double2 rv = ld2(a.r[k] + r);
         rv.x = xsub(rv.x, xmul(w, tv.x));
         rv.y = xsub(rv.y, xmul(w, tv.y));
-        st2(a.x[k] + r, xv);
         st2(a.r[k] + r, rv);
         acc[2 * k] += rv.x * rv.x;
         acc[2 * k + 1] += rv.x * r0.x;
@@ -1299,13 +1303,10 @@ __global__ void __launch_bounds__(256) k_bicg_b2(const SArgs<K> a, SState<K> *st
         }
       } else {
         const float wf = static_cast<float>(omv[k]);
-        const float2 zv = ld2ro(a.fz[k] + r), tv = ld2ro(a.ft[k] + r), r0 = ld2ro(a.fr0[k] + r);
-        float2 xs = ld2(a.fxs[k] + r), rv = ld2(a.fr[k] + r);
-        xs.x = fmaf(wf, zv.x, xs.x);
-        xs.y = fmaf(wf, zv.y, xs.y);
+        const float2 tv = ld2ro(a.ft[k] + r), r0 = ld2ro(a.fr0[k] + r);
+        float2 rv = ld2(a.fr[k] + r);
         rv.x = fmaf(-wf, tv.x, rv.x);
         rv.y = fmaf(-wf, tv.y, rv.y);
-        st2(a.fxs[k] + r, xs);
         st2(a.fr[k] + r, rv);
         acc[2 * k] += static_cast<double>(rv.x) * static_cast<double>(rv.x);
         acc[2 * k + 1] += static_cast<double>(rv.x) * static_cast<double>(r0.x);
@@ -1324,6 +1325,7 @@ __global__ void __launch_bounds__(256) k_bicg_b2(const SArgs<K> a, SState<K> *st
     for (int k = 0; k < K; ++k) {
       st->upd[k] = 0;
       if (!act[k]) continue;
+      st->pend[k] |= kPendOmega;
       const double est = sqrt(sm[2 * k]);
       st->beta[k] = (sm[2 * k + 1] / st->rr0[k]) * (st->alpha[k] / st->omega[k]);
       if (!kMixed) {
@@ -1364,39 +1366,95 @@ __global__ void __launch_bounds__(256) k_bicg_b2(const SArgs<K> a, SState<K> *st
   }
 }
 
-// C: p = r + beta (p - w v) ; z = M p
-template <int K, bool kMixed>
-__global__ void __launch_bounds__(256) k_bicg_c(const SArgs<K> a, SState<K> *st) {
-  if (!st->any) return;
-  int act[K];
-  load_active<K>(st, act);
-  double bv[K], wv[K];
+// What a right-hand side's x += alpha M p + w z adds: the scalars, zero where
+// the term is not due.
+template <typename T>
+struct PendingX {
+  T al, w;
+  bool a, o;
+  template <typename S>
+  __device__ __forceinline__ PendingX(const S *st, int k)
+      : al(static_cast<T>(st->alpha[k])),
+        w(static_cast<T>(st->omega[k])),
+        a(st->pend[k] & kPendAlpha),
+        o(st->pend[k] & kPendOmega) {}
+  __device__ __forceinline__ bool any() const { return a || o; }
+  // x with the due terms added, in the order and rounding of separate updates
+  __device__ __forceinline__ T add(T x, T p, T m, T z) const {
+    if constexpr (sizeof(T) == 8) {
+      if (a) x = xadd(x, xmul(al, xmul(p, m)));
+      if (o) x = xadd(x, xmul(w, z));
+    } else {
+      if (a) x = fmaf(al, m * p, x);
+      if (o) x = fmaf(w, z, x);
+    }
+    return x;
+  }
+};
+
+// reliable update of BiCGSTAB, part 1: x += xs and what is pending (FP64) for
+// the flagged right-hand sides; k_bicg_refresh then clears xs
+template <int K>
+__global__ void __launch_bounds__(256) k_bicg_fold(const SArgs<K> a, SState<K> *st) {
+  if (!st->any_upd) return;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    bv[k] = st->beta[k];
-    wv[k] = st->omega[k];
+    if (!st->upd[k]) continue;
+    const PendingX<float> due(st, k);
+    SFR_FOR_PAIRS(i) {
+      const int r = 2 * i;
+      const float2 xs = ld2(a.fxs[k] + r), p = ld2(a.fp0[k] + r), m = ld2ro(a.m32[k] + r);
+      const float2 z = ld2(a.fz[k] + r);
+      double2 xv = ld2(a.x[k] + r);
+      xv.x += static_cast<double>(due.add(xs.x, p.x, m.x, z.x));
+      xv.y += static_cast<double>(due.add(xs.y, p.y, m.y, z.y));
+      st2(a.x[k] + r, xv);
+    }
   }
-  SFR_FOR_PAIRS(i) {
-    const int r = 2 * i;
+}
+
+// C: x += what is pending ; p = r + beta (p - w v) ; z = M p.  A system that
+// stopped in this iteration takes its x alone.
+template <int K, bool kMixed>
+__global__ void __launch_bounds__(256) k_bicg_c(const SArgs<K> a, SState<K> *st) {
+  using T = typename std::conditional<kMixed, float, double>::type;
+  using T2 = typename std::conditional<kMixed, float2, double2>::type;
+  const int any = st->any;
 #pragma unroll
-    for (int k = 0; k < K; ++k) {
-      if (!act[k]) continue;
-      if (!kMixed) {
-        const double2 rv = ld2ro(a.r[k] + r), q = ld2ro(a.q[k] + r), m = ld2ro(a.m[k] + r);
-        double2 p = ld2(a.p0[k] + r);
-        p.x = xadd(rv.x, xmul(bv[k], xsub(p.x, xmul(wv[k], q.x))));
-        p.y = xadd(rv.y, xmul(bv[k], xsub(p.y, xmul(wv[k], q.y))));
-        st2(a.p0[k] + r, p);
-        st2(a.z[k] + r, make_double2(xmul(p.x, m.x), xmul(p.y, m.y)));
-      } else {
-        const float bf = static_cast<float>(bv[k]);
-        const float wf = static_cast<float>(wv[k]);
-        const float2 rv = ld2ro(a.fr[k] + r), q = ld2ro(a.fq[k] + r), m = ld2ro(a.m32[k] + r);
-        float2 p = ld2(a.fp0[k] + r);
-        p.x = fmaf(bf, fmaf(-wf, q.x, p.x), rv.x);
-        p.y = fmaf(bf, fmaf(-wf, q.y, p.y), rv.y);
-        st2(a.fp0[k] + r, p);
-        st2(a.fz[k] + r, make_float2(m.x * p.x, m.y * p.y));
+  for (int k = 0; k < K; ++k) {
+    const bool act = any && st->active[k];
+    const PendingX<T> due(st, k);
+    if (!act && !due.any()) continue;
+    const T bv = static_cast<T>(st->beta[k]), wv = static_cast<T>(st->omega[k]);
+    T *const x = kMixed ? reinterpret_cast<T *>(a.fxs[k]) : reinterpret_cast<T *>(a.x[k]);
+    T *const p = kMixed ? reinterpret_cast<T *>(a.fp0[k]) : reinterpret_cast<T *>(a.p0[k]);
+    T *const z = kMixed ? reinterpret_cast<T *>(a.fz[k]) : reinterpret_cast<T *>(a.z[k]);
+    const T *const m = kMixed ? reinterpret_cast<T *>(a.m32[k]) : reinterpret_cast<T *>(a.m[k]);
+    const T *const rr = kMixed ? reinterpret_cast<T *>(a.fr[k]) : reinterpret_cast<T *>(a.r[k]);
+    const T *const v = kMixed ? reinterpret_cast<T *>(a.fq[k]) : reinterpret_cast<T *>(a.q[k]);
+    SFR_FOR_PAIRS(i) {
+      const int r = 2 * i;
+      T2 pv = ld2(p + r);
+      const T2 mv = ld2ro(m + r);
+      if (due.any()) {
+        const T2 zv = ld2(z + r);
+        T2 xv = ld2(x + r);
+        xv.x = due.add(xv.x, pv.x, mv.x, zv.x);
+        xv.y = due.add(xv.y, pv.y, mv.y, zv.y);
+        st2(x + r, xv);
+      }
+      if (act) {
+        const T2 rv = ld2ro(rr + r), q = ld2ro(v + r);
+        if constexpr (kMixed) {
+          pv.x = fmaf(bv, fmaf(-wv, q.x, pv.x), rv.x);
+          pv.y = fmaf(bv, fmaf(-wv, q.y, pv.y), rv.y);
+          st2(z + r, make_float2(mv.x * pv.x, mv.y * pv.y));
+        } else {
+          pv.x = xadd(rv.x, xmul(bv, xsub(pv.x, xmul(wv, q.x))));
+          pv.y = xadd(rv.y, xmul(bv, xsub(pv.y, xmul(wv, q.y))));
+          st2(z + r, make_double2(xmul(pv.x, mv.x), xmul(pv.y, mv.y)));
+        }
+        st2(p + r, pv);
       }
     }
   }
@@ -1807,11 +1865,11 @@ cudaError_t build_graph(sfr_system *s, int solver, int precision, int threads, i
       SFR_TRY(add_kernel(body, &bp, (void *)k_bicg_b1<K, true>, gv, threads, p2));
       // the reliable updates as plain kernel nodes that return at once when
       // no right-hand side is due (as in the mixed PCG body)
-      SFR_TRY(add_kernel(body, &bp, (void *)k_fold<K>, gv, threads, pf_sel));
+      SFR_TRY(add_kernel(body, &bp, (void *)k_bicg_fold<K>, gv, threads, p2));
       SFR_TRY(add_kernel(body, &bp, (void *)k_bicg_refresh<K, I>, go, threads, pr1));
       SFR_TRY(add_kernel(body, &bp, const_cast<void *>(a2k), gs, threads, p2, ssm));
       SFR_TRY(add_kernel(body, &bp, (void *)k_bicg_b2<K, true>, gv, threads, p2));
-      SFR_TRY(add_kernel(body, &bp, (void *)k_fold<K>, gv, threads, pf_sel));
+      SFR_TRY(add_kernel(body, &bp, (void *)k_bicg_fold<K>, gv, threads, p2));
       SFR_TRY(add_kernel(body, &bp, (void *)k_bicg_refresh<K, I>, go, threads, pr2));
       SFR_TRY(add_kernel(body, &bp, (void *)k_bicg_c<K, true>, gv, threads, p2));
       SFR_TRY(add_kernel(g, &prev, (void *)k_fold<K>, gv, threads, pf_all));
@@ -1899,11 +1957,11 @@ cudaError_t launch_loop(CachedGraph *cg, int solver, bool mixed, int fused, uint
       for (uint32_t it = 0; it < maxit; ++it) {
         SFR_TRY(cudaLaunchKernel(a1k, dim3(gs), dim3(t), pa, ssm, st));
         k_bicg_b1<K, true><<<gv, t, 0, st>>>(a, ps);
-        k_fold<K><<<gv, t, 0, st>>>(a, ps, 0);
+        k_bicg_fold<K><<<gv, t, 0, st>>>(a, ps);
         k_bicg_refresh<K, I><<<go, t, 0, st>>>(a, ps, 1);
         SFR_TRY(cudaLaunchKernel(a2k, dim3(gs), dim3(t), pa, ssm, st));
         k_bicg_b2<K, true><<<gv, t, 0, st>>>(a, ps);
-        k_fold<K><<<gv, t, 0, st>>>(a, ps, 0);
+        k_bicg_fold<K><<<gv, t, 0, st>>>(a, ps);
         k_bicg_refresh<K, I><<<go, t, 0, st>>>(a, ps, 2);
         k_bicg_c<K, true><<<gv, t, 0, st>>>(a, ps);
       }
