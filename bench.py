@@ -174,6 +174,8 @@ def pcg_alg_bytes(n, nnz_off, iters):
 def pcg_kernel_launches(iters, fused=0):
     # setup, start, three kernels per iteration (fused modes 1-3: one; mode 4:
     # one for the whole loop), post-processing
+    if fused == 5:
+        return 1  # the on-chip kernel
     if fused == 4:
         return 4
     return (1 if fused else 3) * iters + 3
@@ -445,7 +447,8 @@ def run_ours(args):
     achieved = alg / (ms_step * 1e-3) / 1e9
     # the timed solves' engine: the autotuner's choice, or the flags given
     fused = int(tune["headline_fp64"]["fused"]) if tune else int(args.fused)
-    tr = committed_traffic("pcg_fp64_fused_loop_iteration" if fused == 4
+    tr = committed_traffic("pcg_fp64_onchip_iteration" if fused == 5
+                           else "pcg_fp64_fused_loop_iteration" if fused == 4
                            else "pcg_fp64_fused_iteration" if fused else "pcg_fp64_iteration")
     traffic = None
     if tr is not None and tr[1] == "per_iteration_128":
@@ -468,7 +471,11 @@ def run_ours(args):
                                f"permuted + RCM; Jacobi-PCG FP64 to 1e-10 (M-norm)",
                    "rows": N, "nnz_offdiag": nnz, "iterations": iters,
                    "format": "SELL-32 from CSRD: FP64 values, 16-bit column offsets",
-                   "engine": ("CUDA graph, one cooperative kernel for the whole solve "
+                   "engine": ("one cooperative kernel for the whole solve (pcg_grid_kernel: "
+                              "per iteration SpMV with all four products, one exchange, update, "
+                              "publication of p; vectors but p in shared memory as they fit)"
+                              if fused == 5 else
+                              "CUDA graph, one cooperative kernel for the whole solve "
                               "(k_pcg_fused_loop: per iteration SpMV+dot, exchange, x/r/z "
                               "update+dot, exchange, p update, wait on the neighbouring blocks; "
                               "q and z kept in shared memory)" if fused == 4 else
@@ -485,7 +492,8 @@ def run_ours(args):
                      "frac": achieved / peak, "traffic": traffic,
                      "frac_on_traffic": (None if traffic is None
                                          else traffic / (ms_step * 1e-3) / 1e9 / peak),
-                     "kernel": ("k_pcg_fused_loop (one launch per solve)" if fused == 4 else
+                     "kernel": ("pcg_grid_kernel (one launch per solve)" if fused == 5 else
+                                "k_pcg_fused_loop (one launch per solve)" if fused == 4 else
                                 "PCG solve graph (one launch per solve: k_pcg_fused per "
                                 "iteration)" if fused else
                                 "PCG solve graph (one launch per solve: k_pcg_a SpMV+dot, "
