@@ -339,7 +339,7 @@ __device__ __forceinline__ bool pcg_mixed_body(const MixedTeamArgs &a, const Tea
         if (vxs != a.xs + r0) st_vec(a.xs + r0 + lr, vxs[lr]);
       }
       if (static_cast<int>(blockIdx.x) == t.b0 && threadIdx.x == 0) {
-        rt.iters[t.sys] = static_cast<int>(j + 1);
+        rt.put_iters(t.sys, t.round, j + 1);
         *st = MixedState{conv, bnorm, d, rmax, j + 1, refine, resume ? st->t0 : t.t0};
       }
       return false;
@@ -399,7 +399,7 @@ __global__ void __launch_bounds__(kT, kSmThreads / kT)
     over = pcg_mixed_body<I>(a, t, reinterpret_cast<char *>(sm_dyn), smem, sh, round_base(round),
                              round_base(round), t.slices_left > kKeepSlices, states + t.sys, rt, round > 0, round_cap(rt, t, round));
   __syncthreads();
-  end_round(rt, over && static_cast<int>(blockIdx.x) == t.b0, t.sys);
+  end_round(rt, t, over && static_cast<int>(blockIdx.x) == t.b0);
 }
 
 const void *team_kernel(const sfr_system *s, int per_sm) {
@@ -424,7 +424,7 @@ TeamShape team_shape_mixed(const sfr_system *s, int per_sm) {
 }
 
 size_t team_ws_bytes_mixed_team(int n, int grid, int nsys) {
-  return align256((sizeof(MixedState) + 2 * sizeof(int)) * static_cast<size_t>(nsys)) +
+  return align256((sizeof(MixedState) + kRoundInts * sizeof(int)) * static_cast<size_t>(nsys)) +
          align256(sizeof(double) * static_cast<size_t>(n)) +
          4 * align256(sizeof(float) * static_cast<size_t>(n)) +
          align256(sizeof(TeamSlot) * 2 * static_cast<size_t>(grid)) +
@@ -439,7 +439,7 @@ int graph_mixed_team(sfr_system *s, const double *d_b, double *d_x, double tol, 
   const size_t slot_b = align256(sizeof(TeamSlot) * 2 * static_cast<size_t>(plan.grid));
   const size_t tick_b = align256(64 * static_cast<size_t>(plan.grid));
   const size_t state_b =
-      align256((sizeof(MixedState) + 2 * sizeof(int)) * static_cast<size_t>(plan.nsys));
+      align256((sizeof(MixedState) + kRoundInts * sizeof(int)) * static_cast<size_t>(plan.nsys));
   char *base = static_cast<char *>(ws);
   MixedState *states = reinterpret_cast<MixedState *>(base + slot_b + tick_b);
   RoundTable rt = round_table(plan, reinterpret_cast<int *>(states + plan.nsys), ctl);

@@ -344,7 +344,7 @@ __device__ __forceinline__ bool pcg_grid_body(const ChipArgs &a, const TeamPart 
         st->nu_old = sc.nu_old;
         st->j = j + 1;
         if (!resume) st->t0 = t.t0;
-        rt->iters[t.sys] = static_cast<int>(j + 1);
+        rt->put_iters(t.sys, t.round, j + 1);
       }
       return false;
     }
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(kT, kGridThreads / kT)
                                         round > 0, cap);
   }
   __syncthreads();
-  end_round(rt, over && static_cast<int>(blockIdx.x) == t.b0, t.sys);
+  end_round(rt, t, over && static_cast<int>(blockIdx.x) == t.b0);
 }
 
 // ---- cluster form --------------------------------------------------------
@@ -766,7 +766,7 @@ TeamShape team_shape_onchip(const sfr_system *s, int per_sm) {
 }
 
 size_t team_ws_bytes_onchip(int n, int grid, int nsys) {
-  return align256((sizeof(ChipState) + 2 * sizeof(int)) * static_cast<size_t>(nsys)) +
+  return align256((sizeof(ChipState) + kRoundInts * sizeof(int)) * static_cast<size_t>(nsys)) +
          2 * align256(sizeof(double) * static_cast<size_t>(n)) +
          align256(sizeof(TeamSlot) * 2 * static_cast<size_t>(grid)) +
          align256(64 * static_cast<size_t>(grid));
@@ -779,7 +779,7 @@ int graph_team_onchip(sfr_system *s, const double *d_b, double *d_x, double tol,
   const size_t slot_b = align256(sizeof(TeamSlot) * 2 * static_cast<size_t>(plan.grid));
   const size_t tick_b = align256(64 * static_cast<size_t>(plan.grid));
   const size_t state_b =
-      align256((sizeof(ChipState) + 2 * sizeof(int)) * static_cast<size_t>(plan.nsys));
+      align256((sizeof(ChipState) + kRoundInts * sizeof(int)) * static_cast<size_t>(plan.nsys));
   char *base = static_cast<char *>(ws);
   ChipArgs a{};
   a.n = s->n;

@@ -28,7 +28,8 @@ struct TeamPlan {
 TeamShape team_shape(int device, const void *kern, int threads, int per_sm, int slice_bytes,
                      const TeamModel &model);
 
-// done and iters: 2 * plan.nsys ints, zero at first; ctl: 16 words.
+// done_iters: kRoundInts * plan.nsys ints, zero at first; ctl: 16 words.
+constexpr int kRoundInts = 3;
 inline RoundTable round_table(const TeamPlan &plan, int *done_iters, unsigned *ctl) {
   RoundTable rt{};
   rt.sys = plan.systems;

@@ -28,6 +28,7 @@ struct TeamPart {
   int row_end;  // the system's rows end here
   int sys;
   int slices_left;  // a batched launch: slices of the systems of this round
+  unsigned round;   // a batched launch: its round
   unsigned long long t0;  // the block's start (global_ns)
   __device__ __forceinline__ int owner(int row) const {
     const long long B = b1 - b0, ns = count, sl = row / kWarp - first;
@@ -55,10 +56,15 @@ struct TeamModel {
   }
 };
 
+// Blocks make a round's shares each for itself, and one may still be at it
+// when a team of the same round stores that it is done.  So what round r
+// stores, only the rounds after it read: `done` says in which round, and of
+// the two rows of `iters` r reads one and writes the other.  (Every system
+// that is not done has a team in each round, which writes its entry.)
 struct RoundTable {
   const int4 *sys;   // per system {first slice, slices, end row, estimated iterations}
-  int *done;         // per system, set when its result is written
-  int *iters;        // per system, the iterations of the rounds before
+  int *done;         // per system, 1 + the round that wrote its result; 0: none yet
+  int *iters;        // two rows of one entry a system: the iterations of the rounds before
   int nsys;
   int most;          // slices a block can hold
   TeamModel model;
@@ -67,14 +73,27 @@ struct RoundTable {
   unsigned *ctl;     // {round, blocks that finished it, systems done}, zero at first
   int *err;
   cudaGraphConditionalHandle more;  // the WHILE node's condition
+
+  __device__ __forceinline__ bool done_before(int s, unsigned round) const {
+    return static_cast<unsigned>(__ldcg(done + s) - 1) < round;
+  }
+  __device__ __forceinline__ int iters_before(int s, unsigned round) const {
+    return __ldcg(iters + (round & 1u) * nsys + s);
+  }
+  __device__ __forceinline__ void put_done(int s, unsigned round) const {
+    done[s] = static_cast<int>(round + 1u);
+  }
+  __device__ __forceinline__ void put_iters(int s, unsigned round, unsigned n) const {
+    iters[((round + 1u) & 1u) * nsys + s] = static_cast<int>(n);
+  }
 };
 
 // Ends a block's round: the last block to come by counts the round and stops
 // the loop when no system is left (or a wait gave up).
-__device__ __forceinline__ void end_round(const RoundTable &rt, bool over, int sys) {
+__device__ __forceinline__ void end_round(const RoundTable &rt, const TeamPart &t, bool over) {
   if (threadIdx.x != 0) return;
   if (over) {
-    rt.done[sys] = 1;
+    rt.put_done(t.sys, t.round);
     atomicAdd(rt.ctl + 2, 1u);
   }
   __threadfence();
@@ -87,8 +106,9 @@ __device__ __forceinline__ void end_round(const RoundTable &rt, bool over, int s
     cudaGraphSetConditional(rt.more, 0u);
 }
 
-// Shares the grid's blocks over the systems not done so that the slowest
-// team, by the model above and the estimated iterations, takes least.  False
+// Shares the grid's blocks over the systems not done before t.round so that
+// the slowest team, by the model above and the estimated iterations, takes
+// least: from what the rounds before stored, the same in every block.  False
 // when none is left; t.b1 == t.b0 for a block without a team.  The block has
 // at least nsys threads.  scan: two rows of 32 ints.
 __device__ __forceinline__ bool next_teams(const RoundTable &rt, TeamPart &t, int *scan) {
@@ -96,8 +116,8 @@ __device__ __forceinline__ bool next_teams(const RoundTable &rt, TeamPart &t, in
   int4 s = make_int4(0, 0, 0, 1);
   if (i < rt.nsys) {
     s = rt.sys[i];
-    if (__ldcg(rt.done + i)) s.y = 0;
-    s.w = max(s.w - __ldcg(rt.iters + i), s.w / 4 + 1);  // what it may still need
+    if (rt.done_before(i, t.round)) s.y = 0;
+    s.w = max(s.w - rt.iters_before(i, t.round), s.w / 4 + 1);  // what it may still need
   }
   // over the block, in every thread
   auto total = [&](int v) {
@@ -187,6 +207,7 @@ __device__ __forceinline__ TeamPart team_part(const TeamTable &tt, const RoundTa
                                               unsigned round, int *scan) {
   TeamPart t;
   t.t0 = global_ns();
+  t.round = round;
   if (round > 0) {
     if (!next_teams(rt, t, scan)) t.b0 = t.b1 = 0;
     return t;
