@@ -824,13 +824,16 @@ int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double 
   const size_t slot_b = align(sizeof(TeamSlot) * 2 * static_cast<size_t>(sh.grid));
   const size_t tick_b = align(64 * static_cast<size_t>(sh.grid)) + 256;  // + the error word
   const size_t out_b = align(sizeof(SolveOut));
-  // x is written while b is still read: a caller's x that overlaps b gets a
-  // copy of b
-  const uintptr_t xb = reinterpret_cast<uintptr_t>(d_x), bb = reinterpret_cast<uintptr_t>(d_b);
+  // x is written while b and the diagonal are still read: where a caller's x
+  // overlaps one of them, it gets a copy
   const size_t nb = sizeof(double) * static_cast<size_t>(s->n);
-  const bool overlap = xb < bb + nb && bb < xb + nb;
+  const auto under_x = [&](const double *p) {
+    const uintptr_t xb = reinterpret_cast<uintptr_t>(d_x), pb = reinterpret_cast<uintptr_t>(p);
+    return p && xb < pb + nb && pb < xb + nb;
+  };
+  const bool overlap = under_x(d_b), overlap_d = under_x(d_diag);
   int rc = ensure_workspace(s, (sh.cluster ? 0 : 2 * vec + slot_b + tick_b) + out_b +
-                                   (overlap ? vec : 0));
+                                   (overlap ? vec : 0) + (overlap_d ? vec : 0));
   if (rc != SFR_OK) return rc;
   char *base = static_cast<char *>(s->ws.base);
 
@@ -854,6 +857,12 @@ int solve_onchip(sfr_system *s, const double *d_diag, const double *d_b, double 
     if (cudaMemcpyAsync(base, d_b, nb, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
       return SFR_CUDA_ERROR;
     a.b = reinterpret_cast<double *>(base);
+    base += vec;
+  }
+  if (overlap_d) {
+    if (cudaMemcpyAsync(base, d_diag, nb, cudaMemcpyDeviceToDevice, st) != cudaSuccess)
+      return SFR_CUDA_ERROR;
+    a.diag = reinterpret_cast<double *>(base);
     base += vec;
   }
   if (!sh.cluster) {
