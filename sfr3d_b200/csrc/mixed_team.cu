@@ -58,21 +58,6 @@ struct MixedState {
   unsigned long long t0;  // its first round's start (global_ns)
 };
 
-// Hands out a block's dynamic shared memory from the front.
-struct Carve {
-  char *at;
-  int left;
-  template <typename T>
-  __device__ __forceinline__ T *take(int count) {
-    const int bytes = (count * static_cast<int>(sizeof(T)) + 7) & ~7;
-    if (bytes > left) return nullptr;
-    T *p = reinterpret_cast<T *>(at);
-    at += bytes;
-    left -= bytes;
-    return p;
-  }
-};
-
 // At most `cap` iterations of a system, going on from *st when `resume`; true
 // when its solve is over.
 template <typename I>

@@ -410,10 +410,10 @@ __global__ void __launch_bounds__(kT, kGridThreads / kT)
     const int slices = t.s1 - t.s0, rows = slices * kWarp;
     const int left = smem - 4 * (slices + 1);
     const int slots = __ldg(a.sptr + t.s1) - __ldg(a.sptr + t.s0);
-    if (rows * level_bytes(3) + slots * static_cast<int>(8 + sizeof(I)) <= left)
+    if (block_fits(rows, level_bytes(3), slots, 8 + sizeof(I), left))
       over = pcg_grid_body<I, 3, kHold>(a, t, sm_dyn, sh, base, base, st, &rt,
                                         round > 0, cap);
-    else if (rows * level_bytes(2) <= left)
+    else if (block_fits(rows, level_bytes(2), 0, 0, left))
       over = pcg_grid_body<I, 2, kPolicy>(a, t, sm_dyn, sh, base, base, st, &rt,
                                         round > 0, cap);
     else

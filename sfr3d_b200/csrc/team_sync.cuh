@@ -226,6 +226,30 @@ __device__ __forceinline__ TeamPart team_part(const TeamTable &tt, const RoundTa
   return t;
 }
 
+// Whether a block's rows and slots fit `left` bytes of shared memory.  In 64
+// bits: a block of a few hundred rows may have more slots than 2^31 bytes hold.
+__host__ __device__ constexpr bool block_fits(int rows, int row_bytes, int slots, int slot_bytes,
+                                              int left) {
+  return static_cast<long long>(rows) * row_bytes + static_cast<long long>(slots) * slot_bytes <=
+         left;
+}
+
+// Hands out a block's dynamic shared memory from the front.
+struct Carve {
+  char *at;
+  int left;
+  template <typename T>
+  __host__ __device__ __forceinline__ T *take(int count) {
+    const long long bytes =
+        (static_cast<long long>(count) * static_cast<long long>(sizeof(T)) + 7) & ~7ll;
+    if (bytes > left) return nullptr;
+    T *p = reinterpret_cast<T *>(at);
+    at += bytes;
+    left -= static_cast<int>(bytes);
+    return p;
+  }
+};
+
 // Matrix loads under an L2 policy.
 __device__ __forceinline__ double ld_mat(const double *p, uint64_t pol) {
   double v;
