@@ -174,12 +174,12 @@ int sfr_gpu_set_prefetch(sfr_system *s, int32_t rounds);
  * whose p its next SpMV phase gathers.  Solves it
  * does not serve (other solvers, K > 1, mixed precision, or no co-resident
  * shape) take the three-kernel iteration; 0 turns the fused iteration off
- * (three kernels an iteration); other values are SFR_BAD_INPUT.  A handle
- * this was never called for solves FP64 PCG with one right-hand side on the
- * on-chip engine (one launch a solve, one reduction an iteration, the Krylov
+ * (three kernels an iteration); other values are SFR_BAD_INPUT.  Under
+ * the automatic choice (engine 0), a handle this was never called for solves
+ * FP64 PCG with one right-hand side on the on-chip engine (one launch a solve, one reduction an iteration, the Krylov
  * vectors in shared memory; small systems wholly inside one thread-block
  * cluster), or in mode 4 where the system does not fit it; sfr_tune_result
- * reports it as mode 5. */
+ * reports it as mode 5.  Under engine 2 mode 4 is the default. */
 int sfr_gpu_set_fused(sfr_system *s, int32_t mode);
 
 /* Graph engine, BiCGSTAB: 1 stages each warp's SELL slices (slot values and

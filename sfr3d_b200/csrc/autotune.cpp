@@ -228,7 +228,8 @@ extern "C" int sfr_gpu_autotune(sfr_system *s, int32_t solver, int32_t k, const 
   auto measure = [&](size_t from) {
     ms.resize(cands.size(), std::numeric_limits<double>::infinity());
     for (size_t c = from; c < cands.size() && hard == SFR_OK; ++c) {
-      s->engine = cands[c].engine;
+      // on chip: where the automatic choice puts such a solve
+      s->engine = cands[c].engine == 2 && cands[c].fused == kFusedOnChip ? 0 : cands[c].engine;
       s->graph_threads = cands[c].threads ? cands[c].threads : threads0;
       s->graph_spw = cands[c].spw;
       s->graph_pf = cands[c].pf;

@@ -105,8 +105,8 @@ struct sfr_system {
   int32_t graph_spw = 0;         // SELL slices per warp; 0: one wave of resident blocks
   int32_t graph_pf = 0;          // SpMV-phase L2 prefetch distance (rounds); 0: off
   // FP64 PCG, one RHS: 0 three kernels an iteration, 1-4 the fused iteration's
-  // modes, kFusedOnChip the on-chip engine (mode 4 where it does not fit), of
-  // FP64 BiCGSTAB too
+  // modes, kFusedOnChip the on-chip engine under engine 0 (mode 4 where it does
+  // not fit, and under engine 2), of FP64 BiCGSTAB too
   int32_t graph_fused = sfr::kFusedOnChip;
   int32_t graph_stage = 0;       // BiCGSTAB SpMV phases: slices staged in shared memory
   std::vector<sfr::Tuned> tuned; // autotuned choices, used when engine == 0

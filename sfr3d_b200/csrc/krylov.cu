@@ -870,9 +870,10 @@ int enqueue_team_fp64(sfr_system *s, int32_t solver, const double *d_b, double *
              : SFR_CUDA_ERROR;
 }
 
-// BiCGSTAB solves that go to the on-chip engine when they fit it: FP64 under
-// the automatic choice and engine 2, and, under the automatic choice, mixed
-// ones too, in FP64 throughout.  On chip an iteration waits on exchanges and
+// BiCGSTAB solves that go to the on-chip engine when they fit it, under the
+// automatic choice (engine 0, or a tuned entry's): FP64, and, where no entry
+// names an engine, mixed ones too, in FP64 throughout.  On chip an iteration
+// waits on exchanges and
 // gathers, not on bytes, so FP32 inner vectors would gain little, and the
 // reliable updates' FP64 passes fall away.  Mixed kernels against this one, us
 // a solve of one / three systems: 8^3 105 / 180 and 45 / 54, 40^3 226 / 401
@@ -942,13 +943,16 @@ int solve_device(sfr_system *s, int32_t solver, int32_t k, const double *d_diag_
     // automatic choice: a diagonal that is not positive has no Jacobi scaling
     if (rc != SFR_UNSUPPORTED || (engine == 4 && !tuned)) return rc;
   }
-  if ((engine == 0 || engine == 2) && precision == SFR_FP64 && solver == SFR_PCG && k == 1 &&
-      fused == kFusedOnChip) {
+  // on chip under the automatic choice alone: a caller's engine 2 is the graph
+  // engine, with the launch shape, prefetch and staging set for it
+  const bool automatic = s->engine == 0;
+  if (automatic && (engine == 0 || engine == 2) && precision == SFR_FP64 && solver == SFR_PCG &&
+      k == 1 && fused == kFusedOnChip) {
     const int rc = solve_onchip(s, d_diag_k, d_b, d_x, tol, maxit, newx, st, info);
     if (rc != SFR_UNSUPPORTED) return rc;
   }
   int32_t iters0[kMaxK] = {};  // iterations before the engine below
-  if (onchip_bicg_case(s, solver, precision, engine, fused)) {
+  if (automatic && onchip_bicg_case(s, solver, precision, engine, fused)) {
     sfr_solve_info mine[kMaxK];
     const int rc = solve_onchip_bicg(s, k, d_diag_k, d_b, d_x, tol, maxit, newx, st, mine);
     if (rc != SFR_UNSUPPORTED) {
