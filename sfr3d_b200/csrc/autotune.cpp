@@ -168,8 +168,13 @@ extern "C" int sfr_gpu_autotune(sfr_system *s, int32_t solver, int32_t k, const 
   }
   if (cudaSetDevice(s->device) != cudaSuccess) return SFR_CUDA_ERROR;
   const bool own_diag = ad_k == nullptr;
-  const Candidate def{auto_engine(s, solver, k, precision, own_diag), s->graph_threads,
-                      s->graph_spw, s->graph_pf, s->graph_fused};
+  // mixed BiCGSTAB is on chip where its engine has no number
+  const int32_t auto_eng = auto_engine(s, solver, k, precision, own_diag);
+  const bool bicg_chip =
+      solver == SFR_PBICGSTAB &&
+      (precision == SFR_FP64 ? onchip_bicg_fits(s, k, own_diag) : auto_eng == 0);
+  const Candidate def{auto_eng, s->graph_threads, s->graph_spw, s->graph_pf,
+                      bicg_chip ? kFusedOnChip : s->graph_fused};
   if (const Tuned *t = find_tuned(s, solver, k, precision, own_diag)) {
     fill(out, *t, def, 0.0, 0, 1);
     return SFR_OK;
@@ -195,8 +200,7 @@ extern "C" int sfr_gpu_autotune(sfr_system *s, int32_t solver, int32_t k, const 
   if (precision == SFR_FP64 && solver == SFR_PCG && k == 1) {
     for (int mode : {1, 2, 3, 4, kFusedOnChip}) add({2, 256, 0, 0, mode});
   }
-  if (precision == SFR_FP64 && solver == SFR_PBICGSTAB && onchip_bicg_fits(s, k, own_diag))
-    add({2, 256, 0, 0, kFusedOnChip});
+  if (bicg_chip) add({auto_eng, 256, 0, 0, kFusedOnChip});
   add({1, 0, 0, 0, 0});
   if (precision == SFR_MIXED && solver == SFR_PCG && k == 1 && own_diag && resident_fits(s))
     add({4, 0, 0, 0, 0});

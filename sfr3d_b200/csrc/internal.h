@@ -106,7 +106,7 @@ struct sfr_system {
   int32_t graph_pf = 0;          // SpMV-phase L2 prefetch distance (rounds); 0: off
   // FP64 PCG, one RHS: 0 three kernels an iteration, 1-4 the fused iteration's
   // modes, kFusedOnChip the on-chip engine under engine 0 (mode 4 where it does
-  // not fit, and under engine 2), of FP64 BiCGSTAB too
+  // not fit, and under engine 2)
   int32_t graph_fused = sfr::kFusedOnChip;
   int32_t graph_stage = 0;       // BiCGSTAB SpMV phases: slices staged in shared memory
   std::vector<sfr::Tuned> tuned; // autotuned choices, used when engine == 0

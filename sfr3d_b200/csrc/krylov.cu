@@ -871,17 +871,17 @@ int enqueue_team_fp64(sfr_system *s, int32_t solver, const double *d_b, double *
 }
 
 // BiCGSTAB solves that go to the on-chip engine when they fit it, under the
-// automatic choice (engine 0, or a tuned entry's): FP64, and, where no entry
-// names an engine, mixed ones too, in FP64 throughout.  On chip an iteration
-// waits on exchanges and
+// automatic choice (engine 0) or a tuned entry that names it (engine 2 or 0 in
+// mode kFusedOnChip; set_fused is PCG's alone): FP64, and, under engine 0, mixed
+// ones too, in FP64 throughout.  On chip an iteration waits on exchanges and
 // gathers, not on bytes, so FP32 inner vectors would gain little, and the
 // reliable updates' FP64 passes fall away.  Mixed kernels against this one, us
 // a solve of one / three systems: 8^3 105 / 180 and 45 / 54, 40^3 226 / 401
 // and 94 / 109, 60^3 401 / 641 and 151 / 210, 76^3 513 / 984 and 210 / 521,
 // 92^3 of one 768 and 498.
-static bool onchip_bicg_case(const sfr_system *s, int32_t solver, int32_t precision, int32_t engine,
-                      int32_t fused) {
-  return solver == SFR_PBICGSTAB && fused == kFusedOnChip &&
+static bool onchip_bicg_case(int32_t solver, int32_t precision, int32_t engine,
+                             const Tuned *tuned) {
+  return solver == SFR_PBICGSTAB && (!tuned || tuned->fused == kFusedOnChip) &&
          ((precision == SFR_FP64 && (engine == 0 || engine == 2)) ||
           (precision == SFR_MIXED && engine == 0));
 }
@@ -899,8 +899,7 @@ int auto_engine(sfr_system *s, int32_t solver, int32_t k, int32_t precision, boo
   if (resident_case && s->n >= kResidentRows && resident_fits(s)) return 4;
   if (precision == SFR_FP64 && solver == SFR_PCG && k == 1 && s->graph_fused == kFusedOnChip)
     return 2;  // the on-chip engine, at every size
-  if (onchip_bicg_case(s, solver, precision, 0, s->graph_fused) &&
-      onchip_bicg_fits(s, k, own_diag))
+  if (onchip_bicg_case(solver, precision, 0, nullptr) && onchip_bicg_fits(s, k, own_diag))
     return precision == SFR_FP64 ? 2 : 0;
   return s->n >= kGraphEngineRows ? 2 : 1;
 }
@@ -918,16 +917,14 @@ int solve_device(sfr_system *s, int32_t solver, int32_t k, const double *d_diag_
   int engine = s->engine;
   int threads = s->graph_threads, spw = s->graph_spw, pf = s->graph_pf, fused = s->graph_fused;
   const bool resident_case = precision == SFR_MIXED && solver == SFR_PCG && k == 1 && !d_diag_k;
-  bool tuned = false;
-  if (engine == 0) {
-    if (const Tuned *t = find_tuned(s, solver, k, precision, d_diag_k == nullptr)) {
-      engine = t->engine;
-      threads = t->threads;
-      spw = t->spw;
-      pf = t->pf;
-      fused = t->fused;
-      tuned = true;
-    }
+  const Tuned *tuned =
+      engine == 0 ? find_tuned(s, solver, k, precision, d_diag_k == nullptr) : nullptr;
+  if (tuned) {
+    engine = tuned->engine;
+    threads = tuned->threads;
+    spw = tuned->spw;
+    pf = tuned->pf;
+    fused = tuned->fused;
   }
   // the resident engine takes no call without iterations; the persistent one,
   // which has the smaller systems otherwise, does
@@ -952,7 +949,7 @@ int solve_device(sfr_system *s, int32_t solver, int32_t k, const double *d_diag_
     if (rc != SFR_UNSUPPORTED) return rc;
   }
   int32_t iters0[kMaxK] = {};  // iterations before the engine below
-  if (automatic && onchip_bicg_case(s, solver, precision, engine, fused)) {
+  if (automatic && onchip_bicg_case(solver, precision, engine, tuned)) {
     sfr_solve_info mine[kMaxK];
     const int rc = solve_onchip_bicg(s, k, d_diag_k, d_b, d_x, tol, maxit, newx, st, mine);
     if (rc != SFR_UNSUPPORTED) {

@@ -1,5 +1,5 @@
 """What a caller's choice of engine and options selects: engine 2 the graph
-engine's kernels."""
+engine's kernels, set_fused the PCG iteration alone."""
 from __future__ import annotations
 
 import pytest
@@ -75,3 +75,23 @@ def test_tuned_choice_still_reaches_the_on_chip_engine(cuda, tmp_path, monkeypat
         g.set_engine(0)
         assert bits_equal(g.solve_multi(solver, b, tol=TOL)[0], auto)
         g.close()
+
+
+@pytest.mark.parametrize("precision", [sv.FP64, sv.MIXED], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("mode", [0, 4])
+def test_set_fused_concerns_pcg_alone(cuda, precision, mode, tmp_path, monkeypatch):
+    monkeypatch.setenv("SFR_TUNE_CACHE", str(tmp_path / "tune"))
+    s, f = pressure(20), flow((20, 21, 19))
+    g, h = system(s), system(f)
+    x = g.solve(sv.PCG, s.b[0], tol=TOL)[0]
+    y = h.solve_multi(sv.PBICGSTAB, f.b, tol=TOL, precision=precision)[0]
+    g.set_fused(mode)
+    h.set_fused(mode)
+    assert not bits_equal(g.solve(sv.PCG, s.b[0], tol=TOL)[0], x)
+    assert bits_equal(h.solve_multi(sv.PBICGSTAB, f.b, tol=TOL, precision=precision)[0], y)
+    rep = h.autotune(sv.PBICGSTAB, f.b, tol=TOL, precision=precision)
+    assert rep["default_fused"] == 5
+    if rep["fused"] == 5:  # the automatic choice won, and is what runs
+        assert bits_equal(h.solve_multi(sv.PBICGSTAB, f.b, tol=TOL, precision=precision)[0], y)
+    g.close()
+    h.close()
