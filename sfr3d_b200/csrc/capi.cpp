@@ -506,6 +506,9 @@ int transpose_view(sfr_system *s, sfr_system **out) {
   t->engine = s->engine;
   t->graph_threads = s->graph_threads;
   t->graph_spw = s->graph_spw;
+  t->graph_pf = s->graph_pf;
+  t->graph_fused = s->graph_fused;
+  t->graph_stage = s->graph_stage;
   if (t->comp_stale && s->values_set) {
     rc = sfr::row_compensation(t, t->A, t->stream);
     if (rc != SFR_OK) return rc;

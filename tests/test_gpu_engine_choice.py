@@ -1,5 +1,6 @@
 """What a caller's choice of engine and options selects: engine 2 the graph
-engine's kernels, set_fused the PCG iteration alone."""
+engine's kernels, set_fused the PCG iteration alone, and the transposed
+system's solves run as the system's own."""
 from __future__ import annotations
 
 import pytest
@@ -95,3 +96,19 @@ def test_set_fused_concerns_pcg_alone(cuda, precision, mode, tmp_path, monkeypat
         assert bits_equal(h.solve_multi(sv.PBICGSTAB, f.b, tol=TOL, precision=precision)[0], y)
     g.close()
     h.close()
+
+
+@pytest.mark.parametrize("engine", [0, 2])
+@pytest.mark.parametrize("fused", [None, 0, 3, 4])
+def test_transposed_solves_run_as_the_system_does(cuda, engine, fused):
+    """A symmetric system is its own transpose, entry for entry, so the same
+    engine in the same mode gives the same bits."""
+    s = pressure(18)
+    g = system(s)
+    g.set_engine(engine)
+    if fused is not None:
+        g.set_fused(fused)
+    x, info = g.solve(sv.PCG, s.b[0], tol=TOL)
+    xt, it = g.solve_transpose(sv.PCG, s.b[0], tol=TOL)
+    assert bits_equal(x, xt) and info.iters == it.iters
+    g.close()
