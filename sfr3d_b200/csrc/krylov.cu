@@ -948,7 +948,10 @@ int solve_device(sfr_system *s, int32_t solver, int32_t k, const double *d_diag_
     const int rc = solve_onchip(s, d_diag_k, d_b, d_x, tol, maxit, newx, st, info);
     if (rc != SFR_UNSUPPORTED) return rc;
   }
-  int32_t iters0[kMaxK] = {};  // iterations before the engine below
+  // what a solve took before the engine below
+  int32_t iters0[kMaxK] = {};
+  double seconds0 = 0.0;
+  const uint32_t cap = maxit;
   if (automatic && onchip_bicg_case(solver, precision, engine, tuned)) {
     sfr_solve_info mine[kMaxK];
     const int rc = solve_onchip_bicg(s, k, d_diag_k, d_b, d_x, tol, maxit, newx, st, mine);
@@ -964,13 +967,35 @@ int solve_device(sfr_system *s, int32_t solver, int32_t k, const double *d_diag_
         return rc;
       }
       newx = 0;
-      for (int i = 0; i < k; ++i) iters0[i] = mine[i].iters;
+      seconds0 = mine[0].seconds;
+      uint32_t most = 0;
+      for (int i = 0; i < k; ++i) {
+        iters0[i] = mine[i].iters;
+        most = std::max(most, static_cast<uint32_t>(mine[i].iters));
+      }
+      if (most >= cap) {  // nothing is left of the call's iterations
+        for (int i = 0; i < k; ++i)
+          if (!(mine[i].norm_r < mine[i].conv)) {
+            mine[i].status = SFR_MAXIT;
+            mine[i].iters = mine[i].inner_iters = static_cast<int32_t>(cap + 1);
+          }
+        if (info) std::copy(mine, mine + k, info);
+        return SFR_MAXIT;
+      }
+      maxit -= most;
     }
   }
   if (fused == kFusedOnChip) fused = 4;
   if (engine == 0 || engine == 4) engine = s->n >= kGraphEngineRows ? 2 : 1;
   const auto total = [&](int rc) {
-    for (int i = 0; i < k && info && rc >= 0; ++i) info[i].iters += iters0[i];
+    if (iters0[0] == 0 || !info || rc < 0) return rc;
+    for (int i = 0; i < k; ++i) {
+      info[i].iters += iters0[i];
+      info[i].inner_iters += iters0[i];
+      info[i].seconds += seconds0;
+      if (info[i].status == SFR_MAXIT)  // counted as a call that runs into its cap is
+        info[i].iters = info[i].inner_iters = static_cast<int32_t>(cap + 1);
+    }
     return rc;
   };
   if (engine == 2 || engine == 3)
