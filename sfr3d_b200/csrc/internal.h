@@ -26,6 +26,7 @@ struct HostSell {
   int32_t bandwidth = 0;
   int32_t max_width = 0;
   int64_t nnz = 0;  // real (non-padded) off-diagonal slots
+  int64_t far = 0;  // ... whose column is more than n / 16 rows away
 };
 
 // Validates the reference layout and builds the SELL copy of A (and, when
@@ -45,6 +46,10 @@ struct DevSell {
   double *val = nullptr;  // FP64 values
   float *val32 = nullptr; // FP32 copy (mixed precision)
   int32_t max_width = 0;  // slots of the widest slice
+  // Share of the real slots whose column is more than n / 16 rows away: 0 on a
+  // numbered mesh (also where a few couplings go far), 0.88 without numbering.
+  float far_share = 0.f;
+  bool far() const { return far_share > 0.4f; }
 };
 
 struct SolveOut;  // device-side result record (krylov.cu)

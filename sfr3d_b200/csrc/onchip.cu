@@ -676,6 +676,10 @@ bool ready(const Shape &sh, int device) {
 // sixteen SMs' arithmetic costs more than the grid form's slower exchange:
 // 24^3 (27 slices a block) 3.12 us an iteration against 3.75, 28^3 (43) 3.75
 // against 4.08, 32^3 (64) 5.8 against 4.26.
+// Without numbering (DevSell::far) most gathers go to other blocks, lane by
+// lane: up to eight slices a block only.  16^3 cells in random order 5.3 us an
+// iteration in the cluster and 3.9 in the grid form, 20^3 7.6 and 4.7, 24^3 11.0
+// and 4.9, 29^3 16.9 and 5.6 (in order 3.9 and 4.4); 10^3 to 14^3 as good.
 constexpr int kClusterBlockSlices = 8, kClusterSlices = 48;
 
 bool cluster_shape(const sfr_system *s, Shape *sh) {
@@ -683,7 +687,7 @@ bool cluster_shape(const sfr_system *s, Shape *sh) {
   int c = 1;
   while (c < kMaxCluster && (ns + c - 1) / c > kClusterBlockSlices) c *= 2;
   const int slices = (ns + c - 1) / c, rows = slices * kWarp;
-  if (slices > kClusterSlices) return false;
+  if (slices > (s->A.far() ? kClusterBlockSlices : kClusterSlices)) return false;
   const size_t limit = static_cast<size_t>(smem_optin(s->device)) - kClusterStatic;
   for (bool vecs : {true, false}) {
     const size_t b = cluster_smem(rows, static_cast<int64_t>(rows) * s->A.max_width, slices, vecs);
