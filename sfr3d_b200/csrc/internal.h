@@ -12,6 +12,8 @@
 namespace sfr {
 
 constexpr int kWarpHost = 32;  // rows per SELL slice (one warp)
+// automatic engine choice: the graph engine from this many rows up
+constexpr int kGraphEngineRows = 100000;
 constexpr int kFusedOnChip = 5;  // sfr_system::graph_fused: the on-chip engine
 
 // SELL-32 layout built on the host from one of the reference's layouts.

@@ -615,8 +615,6 @@ int stat_grid(int device, int64_t n) {
 
 namespace {
 
-// automatic engine choice: the graph engine from this many rows up
-constexpr int kGraphEngineRows = 100000;
 // mixed PCG: the resident engine from this many rows up.  An iteration of an
 // 8^3 box takes 2.0 us there and 8.9 us in the persistent kernel, of a 16^3 box
 // 3.6 and 7.8, of a 40^3 box 5.5 and 9.3, of a 56^3 box 6.6 and 14.  Below, a

@@ -443,13 +443,45 @@ struct Shape {
   size_t smem = 0;
 };
 
-// What an iteration reads past shared memory may be this much, of the 126 MB
-// of L2; past it the streaming engine's kernels, with four times the warps,
-// hide HBM better.  Device time, this kernel and those: 72^3 of 3 systems (67
-// MB) 361 and 717 us, 96^3 of 1 (90 MB) 565 and 741, 88^3 of 2 (101 MB) 939
-// and 970, 80^3 of 3 (108 MB) 868 and 976; 104^3 of 1 (121 MB) 1229 and 953,
-// 88^3 of 3 (142 MB) 1384 and 1356.
+// What an iteration reads past shared memory may be this much of the 126 MB of
+// L2, or, from kGraphEngineRows rows on, what live_line says: past it this
+// kernel waits on HBM with too few loads in flight, and the streaming engine,
+// with four times the warps, hides it better.  (Below, the other choice is the
+// persistent kernel, whose five barriers an iteration cost more: 40,000 rows of
+// 100 slots, three systems, 38 us and 133.)
 constexpr size_t kLiveBytes = 110 << 20;
+
+// us an iteration, this kernel and the streaming engine, FP64, by the live
+// bytes in MB and K (m: against the mixed streaming solve):
+//   K 1  94^3 cells (76) 43, 73; 96^3 (88) 56, 70; 100^3 (100) 75, 80; 102^3
+//        (115) 103, 82; 100,000 rows of 100 slots (102) 68, 74 (m 71); 250,000
+//        of 40 (104) 93, 71
+//   K 2  80^3 (68) 51, 85; 84^3 (88) 75, 95; 86^3 (94) 87, 94; 88^3 (101) 109,
+//        101; 27-point 66^3 (80) 48, 80; 68^3 (93) 100, 96; 100,000 rows of 100
+//        slots (102) 152, 84; 600,000 of 8 (101) 100, 86
+//   K 3  76^3 (83) 63, 105; 27-point 64^3 (88) 81, 93; 400,000 rows of 12 slots
+//        (99) 89, 94; 225,000 of 40 (103) 94, 96; 300,000 of 24 (103) 92, 88;
+//        100,000 of 100 (103) 117, 96.  Where the operator is a third at most,
+//        what the streaming kernels move of vectors weighs more: 78^3 (101) 97,
+//        117; 80^3 (109) 99, 111; 82^3 (117) 114, 122.
+// Unnumbered meshes (DevSell::far; with kFarSmem): 72^3 of 3 (75) 87, 124; 80^3
+// of 2 (82) 98, 111; 92^3 of 1 (87) 76, 90; 96^3 of 1 (106) 96, 94; 84^3 of 2
+// (95) 125, 124; random rows of 20, 250,000 of 2 (96) 165, 148.
+size_t live_line(const sfr_system *s, int k, size_t op, size_t live) {
+  if (s->n < kGraphEngineRows) return kLiveBytes;
+  if (s->A.far()) return 94000000;
+  if (k == 3) return 3 * op <= live ? kLiveBytes : 102500000;
+  return k == 1 ? 100000000 : 95000000;
+}
+
+// Scattered gathers in flight hold a line of L1 each.  Up to this much shared
+// memory a block (static and the system's 1 KB included: the 196 KB carve-out)
+// leaves 60 KB of L1, the next carve-out 28.  Cells in random order, us an
+// iteration with 190 KB at most and with all of it: 52^3 of 3 37 and 54, 60^3 of
+// 3 50 and 78, 64^3 of 2 42 and 66, 84^3 of 1 47 and 74, 88^3 of 1 53 and 84
+// (the streaming engine: 72, 88, 71, 74 and 80).  Numbered, the vectors that
+// leave cost more than the L1 gives: 76^3 of 3 63 with all, 75 without.
+constexpr size_t kFarSmem = (196 << 10) - 1024;
 
 template <typename I, int K>
 bool shape_of(const sfr_system *s, bool own_diag, Shape *sh) {
@@ -457,7 +489,8 @@ bool shape_of(const sfr_system *s, bool own_diag, Shape *sh) {
   if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device) !=
       cudaSuccess)
     return false;
-  const size_t limit = static_cast<size_t>(optin) - kStatic;
+  const size_t most = static_cast<size_t>(optin) - kStatic;
+  const size_t limit = s->A.far() ? std::min(most, kFarSmem - kStatic) : most;
   const int ns = s->A.nslices;
   const int g = std::max(1, std::min(num_sms(s->device), (ns + kBlockSlices - 1) / kBlockSlices));
   const int slices = (ns + g - 1) / g;
@@ -471,10 +504,10 @@ bool shape_of(const sfr_system *s, bool own_diag, Shape *sh) {
   const bool core = base + kCoreVecs * vec <= limit;
   sh->on_chip = static_cast<int>(std::min<size_t>(kVecs, (limit - base) / vec));
   sh->smem = base + sh->on_chip * vec;
-  const size_t live =
-      (hold ? 0 : s->A.nslots * (8 + sizeof(I))) +
-      sizeof(double) * static_cast<size_t>(s->n) * ((own_diag ? 1 : K) + K * (1 + kVecs - sh->on_chip));
-  if (live > kLiveBytes) return false;
+  const size_t op = hold ? 0 : s->A.nslots * (8 + sizeof(I));
+  const size_t live = op + sizeof(double) * static_cast<size_t>(s->n) *
+                               ((own_diag ? 1 : K) + K * (1 + kVecs - sh->on_chip));
+  if (live > live_line(s, K, op, live)) return false;
   sh->grid = g;
   // a thread watches a block in neighbour_wait
   sh->threads = std::max((g + kWarp - 1) / kWarp * kWarp,
@@ -491,7 +524,7 @@ bool shape_of(const sfr_system *s, bool own_diag, Shape *sh) {
   if (it != known.end()) return it->second;
   const bool ok =
       cudaFuncSetAttribute(sh->kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(limit)) == cudaSuccess;
+                           static_cast<int>(most)) == cudaSuccess;
   if (!ok) (void)cudaGetLastError();  // the refusal is not a later call's error
   known[key] = ok;
   return ok;
