@@ -388,8 +388,17 @@ int run(sfr_batch *b, int32_t solver, double tol, uint32_t maxit, int32_t newx,
 
 }  // namespace
 
+// The SM's shared memory that a batch of unnumbered systems uses at most: the
+// carve-out that leaves 92 KB of L1, where the lines of its scattered gathers
+// in flight live.  With all 228 KB, with 196, 164 and 132, ms a solve, mixed and
+// FP64: 3 boxes of 90^3 in random order 147, 83, 71, 68 and 130, 76, 68, 65; 8 of
+// 48^3 27.9, 17.7, 15.7, 15.4 and 24.8, 14.9, 13.4, 15.7; one of 110^3 80, 60,
+// 52, 54 and 88, 58, 54, 52 (the persistent kernels: 112 and 128, 28.1 and 28.6,
+// 82 and 96).
+constexpr int kFarSmem = 164 << 10;
+
 TeamShape team_shape(int device, const void *kern, int threads, int per_sm, int slice_bytes,
-                     const TeamModel &model) {
+                     const TeamModel &model, bool far) {
   TeamShape sh;
   sh.per_sm = per_sm;
   sh.threads = threads;
@@ -402,10 +411,12 @@ TeamShape team_shape(int device, const void *kern, int threads, int per_sm, int 
       cudaDeviceGetAttribute(&block, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) !=
           cudaSuccess)
     return sh;
-  const int smem =
-      std::min(sm / per_sm - 1024, block) - static_cast<int>((sizeof(TeamShared) + 255) / 256 * 256);
+  constexpr int kStatic = (sizeof(TeamShared) + 255) / 256 * 256;
+  const int most = std::min(sm / per_sm - 1024, block) - kStatic;
+  const int smem = far ? std::min(most, kFarSmem / per_sm - 1024 - kStatic) : most;
+  // the kernel's limit is one for all batches
   if (smem <= 64 ||
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) !=
           cudaSuccess ||
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads,
                                                     static_cast<size_t>(smem)) != cudaSuccess ||
@@ -504,6 +515,8 @@ int sfr_gpu_batch_create(int32_t nsys, const int32_t *neq, const int32_t *nad,
     }
     cat.bandwidth = std::max(cat.bandwidth, h.bandwidth);
     cat.max_width = std::max(cat.max_width, h.max_width);
+    cat.nnz += h.nnz;
+    cat.far += h.far;
     rows += static_cast<int64_t>(h.nslices) * sfr::kWarpHost;
     slices += h.nslices;
     src += ns;

@@ -405,7 +405,7 @@ size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 // slices 3.4.
 TeamShape team_shape_mixed(const sfr_system *s, int per_sm) {
   return team_shape(s->device, team_kernel(s, per_sm), kSmThreads / per_sm, per_sm, kWarp * 4 + 4,
-                    TeamModel{2.5f, 7.5f, 0.12f});
+                    TeamModel{2.5f, 7.5f, 0.12f}, s->A.far());
 }
 
 size_t team_ws_bytes_mixed_team(int n, int grid, int nsys) {

@@ -766,7 +766,7 @@ const void *team_kernel(const sfr_system *s, int per_sm) {
 // slices 2.4.
 TeamShape team_shape_onchip(const sfr_system *s, int per_sm) {
   return team_shape(s->device, team_kernel(s, per_sm), kGridThreads / per_sm, per_sm,
-                    kWarp * level_bytes(0) + 4, TeamModel{0.9f, 4.5f, 0.1f});
+                    kWarp * level_bytes(0) + 4, TeamModel{0.9f, 4.5f, 0.1f}, s->A.far());
 }
 
 size_t team_ws_bytes_onchip(int n, int grid, int nsys) {

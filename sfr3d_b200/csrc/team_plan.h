@@ -24,9 +24,9 @@ struct TeamPlan {
 };
 
 // The shape of `kern` with `per_sm` blocks of `threads` an SM, of which a
-// slice takes slice_bytes at least.
+// slice takes slice_bytes at least; far: for unnumbered systems (DevSell::far).
 TeamShape team_shape(int device, const void *kern, int threads, int per_sm, int slice_bytes,
-                     const TeamModel &model);
+                     const TeamModel &model, bool far);
 
 // done_iters: kRoundInts * plan.nsys ints, zero at first; ctl: 16 words.
 constexpr int kRoundInts = 3;
