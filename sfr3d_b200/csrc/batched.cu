@@ -199,6 +199,30 @@ std::vector<int> share_by_model(const sfr_batch *b, const TeamShape &sh) {
   return nb;
 }
 
+// The time of an on-chip launch's first round, in us, of teams predicted to
+// take t[s] us on nb[s] blocks.  Up to `share` of the slowest team's; less where
+// a quarter of the blocks are predicted idle before, a quarter past that time
+// (predictions are rough), so that the next round gives those blocks to the
+// teams still at work: 112^3 beside 63 boxes of 8^3, which hold 43 % of the
+// blocks for 0.3 ms, 31 ms mixed (share alone 44 to 62, the persistent kernels
+// 44) and 29 FP64 (50, 99); 200 boxes of 4 to 40 cells 12.3 and 10.3 (16.2 and
+// 16.6).  An eighth costs batches of small boxes 4 to 7 %.
+double first_round(const std::vector<double> &t, const std::vector<int> &nb, double share) {
+  const int S = static_cast<int>(nb.size());
+  std::vector<int> order(S);
+  int64_t grid = 0, idle = 0;
+  double longest = 0.0;
+  for (int s = 0; s < S; ++s) {
+    order[s] = s;
+    grid += nb[s];
+    longest = std::max(longest, t[s]);
+  }
+  std::sort(order.begin(), order.end(), [&](int a, int b) { return t[a] < t[b]; });
+  for (int s : order)
+    if (4 * (idle += nb[s]) >= grid) return std::min(share * longest, 1.25 * t[s]);
+  return share * longest;
+}
+
 // Install a launch plan: team s gets nb[s] blocks (b->team_blocks when set
 // by the autotuner, else shares of the work weights).
 int plan(sfr_batch *b, int32_t solver, int32_t precision) {
@@ -248,18 +272,20 @@ int plan(sfr_batch *b, int32_t solver, int32_t precision) {
   const int grid = static_cast<int>(blocks.size());
   const std::vector<double> est = estimates(b);
   std::vector<int4> systems(S);
+  std::vector<double> us(S);
   double longest = 0.0;
   for (int s = 0; s < S; ++s) {
     systems[s] = make_int4(b->slice_off[s], b->nslices[s], b->row_off[s] + b->n[s],
                            static_cast<int>(std::min(est[s], 1e9)));
-    longest = std::max(longest, est[s] * shape.model.us(b->nslices[s], nb[s]));
+    us[s] = est[s] * shape.model.us(b->nslices[s], nb[s]);
+    longest = std::max(longest, us[s]);
   }
   // The first round's time, as a share of what the slowest team is predicted
   // to take, then a quarter a round.  FP64, all of it: 24 small boxes 4.9 ms,
   // half 5.7 (a re-plan costs the small teams more than it gives).  Mixed,
   // half: 64 uneven boxes 72 ms (a quarter 66, all 88, one round 176), small
   // batches 4.5 to 6.5 ms (all 3.5 to 5.6).
-  b->round_us = static_cast<float>((e == kChipMixed ? 0.5 : 1.0) * longest);
+  b->round_us = static_cast<float>(first_round(us, nb, e == kChipMixed ? 0.5 : 1.0));
   b->round_us_later = static_cast<float>(0.25 * longest);
   if (cudaMemcpy(b->d_systems, systems.data(), sizeof(int4) * S, cudaMemcpyHostToDevice) !=
       cudaSuccess)
