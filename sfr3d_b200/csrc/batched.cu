@@ -114,6 +114,18 @@ std::vector<int> least_blocks(const sfr_batch *b, const TeamShape &sh) {
   return nb;
 }
 
+// Slices of which a block of the mixed teams' has room for `vecs` FP32 vectors
+// and the slice pointers.
+int mixed_slices(const TeamShape &sh, int vecs) {
+  return (static_cast<int>(sh.smem) - 32) / (kWarpHost * 4 * vecs + 4);
+}
+
+// Mixed batches too large for the teams to hold q and r in shared memory stay
+// with the persistent kernels, whose more warps stream the rest better: 3 boxes
+// of 112^3 (131,712 slices) 130 ms and 142 on teams, 4 177 and 195, 6 of 96^3
+// 145 and 160, 8 of 62 to 115 cells 170 and 184; 4 of 96^3 (110,592, q and r
+// held) 92 and 79.
+//
 // One block an SM while the systems are at most half as many (96^3 alone:
 // 14.6 us an iteration against 17.5 with two blocks an SM; 64 mixed boxes of
 // 8 to 96 cells 66 ms against 67), else two: twice the teams, finer shares.
@@ -127,7 +139,8 @@ Engine pick_engine(const sfr_batch *b, int32_t solver, int32_t precision, TeamSh
     if (per_sm == 1 && 2 * b->nsys > num_sms(b->device)) continue;
     int64_t total = 0;
     for (int v : least_blocks(b, sh)) total += v;
-    if (sh.blocks > 0 && b->nsys <= kMaxTeams && total <= sh.blocks) {
+    if (sh.blocks > 0 && b->nsys <= kMaxTeams && total <= sh.blocks &&
+        !(e == kChipMixed && b->cat.A.nslices > sh.blocks * mixed_slices(sh, 2))) {
       *shape = sh;
       return e;
     }
