@@ -101,6 +101,24 @@ std::vector<int> share_by_weight(const sfr_batch *b, int gmax) {
   return nb;
 }
 
+// The SM's shared memory that a batch of unnumbered systems uses at most: the
+// carve-out that leaves 92 KB of L1, where the lines of its scattered gathers
+// in flight live.  With all 228 KB, with 196, 164 and 132, ms a solve, mixed and
+// FP64: 3 boxes of 90^3 in random order 147, 83, 71, 68 and 130, 76, 68, 65; 8 of
+// 48^3 27.9, 17.7, 15.7, 15.4 and 24.8, 14.9, 13.4, 15.7; one of 110^3 80, 60,
+// 52, 54 and 88, 58, 54, 52 (the persistent kernels: 112 and 128, 28.1 and 28.6,
+// 82 and 96).
+constexpr int kFarSmem = 164 << 10;
+// ... and mixed teams that hold their vectors in it (plan).
+constexpr int kMixedSmem = 196 << 10;
+
+// A block's dynamic shared memory where the SM's is `sm` bytes: less the team
+// kernels' static shared memory and the 1 KB the system takes of each block.
+size_t team_smem(int sm, int per_sm) {
+  constexpr int kStatic = (sizeof(TeamShared) + 255) / 256 * 256;
+  return static_cast<size_t>(std::max(0, sm / per_sm - 1024 - kStatic));
+}
+
 // What runs a batch: the on-chip teams (PCG: onchip.cu in FP64, mixed_team.cu
 // in mixed precision) where every system has room there, else the persistent
 // kernels.
@@ -268,6 +286,25 @@ int plan(sfr_batch *b, int32_t solver, int32_t precision) {
   total = 0;
   for (int v : nb) total += v;
   b->blocks_of = nb;
+  // The carve-out below the largest leaves 60 KB of L1 for 28, where every team
+  // holds in it what it holds in all of it, or q, r and xs: 2 boxes of 96^3 42.0
+  // -> 39.4 ms (the persistent kernels 37.9), of 80^3 16.8 -> 14.8, 8 of 48^3 9.3
+  // -> 8.3.  Teams that lose more lose time: r, 2 boxes of 128^3 144 -> 158; the
+  // operator, 148 of 12^3 0.80 -> 1.02, 16 of 32^3 4.5 -> 5.0.
+  if (e == kChipMixed) {
+    TeamShape small = shape;
+    small.smem = std::min(shape.smem, team_smem(kMixedSmem, shape.per_sm));
+    small.most = mixed_slices(small, 1);
+    // all of a slice: its rows' vectors and its slots
+    const int whole = kWarpHost * (24 + b->cat.A.max_width * (b->cat.A.off ? 6 : 8)) + 4;
+    const auto room = [&](const TeamShape &sh) { return static_cast<int>(sh.smem - 32) / whole; };
+    bool same = true;
+    for (int s = 0; s < S; ++s) {
+      const int w = (b->nslices[s] + nb[s] - 1) / nb[s];
+      same = same && w <= mixed_slices(small, 3) && (w <= room(small) || w > room(shape));
+    }
+    if (same) shape = small;
+  }
   std::vector<int4> blocks;
   std::vector<int2> sys;
   blocks.reserve(total);
@@ -427,44 +464,31 @@ int run(sfr_batch *b, int32_t solver, double tol, uint32_t maxit, int32_t newx,
 
 }  // namespace
 
-// The SM's shared memory that a batch of unnumbered systems uses at most: the
-// carve-out that leaves 92 KB of L1, where the lines of its scattered gathers
-// in flight live.  With all 228 KB, with 196, 164 and 132, ms a solve, mixed and
-// FP64: 3 boxes of 90^3 in random order 147, 83, 71, 68 and 130, 76, 68, 65; 8 of
-// 48^3 27.9, 17.7, 15.7, 15.4 and 24.8, 14.9, 13.4, 15.7; one of 110^3 80, 60,
-// 52, 54 and 88, 58, 54, 52 (the persistent kernels: 112 and 128, 28.1 and 28.6,
-// 82 and 96).
-constexpr int kFarSmem = 164 << 10;
-
 TeamShape team_shape(int device, const void *kern, int threads, int per_sm, int slice_bytes,
                      const TeamModel &model, bool far) {
   TeamShape sh;
   sh.per_sm = per_sm;
   sh.threads = threads;
   sh.model = model;
-  // an SM's shared memory over its blocks, each with the kernel's static
-  // shared memory and the 1 KB the system takes
   int sm = 0, block = 0, occ = 0;
   if (cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device) !=
           cudaSuccess ||
       cudaDeviceGetAttribute(&block, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) !=
           cudaSuccess)
     return sh;
-  constexpr int kStatic = (sizeof(TeamShared) + 255) / 256 * 256;
-  const int most = std::min(sm / per_sm - 1024, block) - kStatic;
-  const int smem = far ? std::min(most, kFarSmem / per_sm - 1024 - kStatic) : most;
+  const size_t most = std::min(team_smem(sm, per_sm), team_smem(block + 1024, 1));
+  const size_t smem = far ? std::min(most, team_smem(kFarSmem, per_sm)) : most;
   // the kernel's limit is one for all batches
   if (smem <= 64 ||
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most) !=
-          cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads,
-                                                    static_cast<size_t>(smem)) != cudaSuccess ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           static_cast<int>(most)) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem) != cudaSuccess ||
       occ < per_sm) {
     (void)cudaGetLastError();  // the refusal is not a later call's error
     return sh;
   }
-  sh.smem = static_cast<size_t>(smem);
-  sh.most = (smem - 32) / slice_bytes;
+  sh.smem = smem;
+  sh.most = (static_cast<int>(smem) - 32) / slice_bytes;
   // neighbour_wait watches one block a thread
   sh.blocks = std::min(threads, per_sm * num_sms(device));
   return sh;
