@@ -10,10 +10,13 @@
 // the update is about to produce (predict-and-recompute CG: Chen & Carson,
 // SIAM J. Matrix Anal. Appl. 2020).  The next SpMV phase recomputes nu from
 // the residual it holds, so alpha and the stopping test always use the
-// measured product, never the predicted one; nu' only shapes beta, where a
-// rounding error of a few units in the last place costs nothing but a little
-// conjugacy.  An iteration is then SpMV, exchange, update, publication of p:
-// two synchronisations instead of three, and no vector but p leaves the chip.
+// measured product, never the predicted one; nu' only shapes beta, formed as
+// 1 - 2 delta / mu + alpha gamma / mu: right to a few eps in absolute terms, so
+// that a step which takes (r, z) down by many orders leaves beta few digits or
+// none.  p then keeps a few eps of the old direction beside a z many orders
+// larger than that, and the solve goes on as the reference's (a right-hand side
+// of one eigenvector and 1e-11 of noise: the same count of iterations).  An
+// iteration is then SpMV, exchange, update, publication of p: two synchronisations instead of three, and no vector but p leaves the chip.
 // Every SpMV row keeps the reference's rounding and order (diagonal product,
 // then each slot).  A solve runs one SpMV phase beyond its last update, the
 // one that measures the residual it stops on.
