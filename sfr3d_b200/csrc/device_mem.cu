@@ -114,7 +114,7 @@ int upload_sell(const HostSell &h, DevSell *d, int64_t *bytes) {
   d->nslices = h.nslices;
   d->nslots = h.sptr.empty() ? 0 : h.sptr.back();
   d->max_width = h.max_width;
-  d->far_share = h.nnz > 0 ? static_cast<float>(h.far) / static_cast<float>(h.nnz) : 0.f;
+  d->far_share = h.far_of > 0 ? static_cast<float>(h.far) / static_cast<float>(h.far_of) : 0.f;
   if (upload(&d->sptr, h.sptr, bytes) != cudaSuccess) return SFR_CUDA_ERROR;
   if (upload(&d->col, h.col, bytes) != cudaSuccess) return SFR_CUDA_ERROR;
   if (upload(&d->src, h.src, bytes) != cudaSuccess) return SFR_CUDA_ERROR;

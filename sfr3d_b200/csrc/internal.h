@@ -28,7 +28,8 @@ struct HostSell {
   int32_t bandwidth = 0;
   int32_t max_width = 0;
   int64_t nnz = 0;  // real (non-padded) off-diagonal slots
-  int64_t far = 0;  // ... whose column is more than n / 16 rows away
+  // of every 61st row, the slots whose column is more than n / 16 rows away
+  int64_t far = 0, far_of = 0;
 };
 
 // Validates the reference layout and builds the SELL copy of A (and, when

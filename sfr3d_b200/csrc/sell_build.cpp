@@ -56,7 +56,7 @@ bool to_sell(int32_t n, const RowLists &rl, HostSell *h) {
   h->col.assign(nslots, 0);
   h->src.assign(nslots, -1);
   int32_t band = 0;
-  int64_t nnz = 0, far = 0;
+  int64_t nnz = 0;
   for (int32_t s = 0; s < h->nslices; ++s) {
     const int32_t base = h->sptr[s];
     const int32_t w = (h->sptr[s + 1] - base) / kWarpHost;
@@ -69,9 +69,7 @@ bool to_sell(int32_t n, const RowLists &rl, HostSell *h) {
           const int32_t c = rl.col[rl.ptr[r] + k];
           h->col[e] = c;
           h->src[e] = rl.src[rl.ptr[r] + k];
-          const int32_t reach = c > r ? c - r : r - c;
-          band = std::max(band, reach);
-          far += reach > n / 16;
+          band = std::max(band, c > r ? c - r : r - c);
           ++nnz;
         } else {
           h->col[e] = r < n ? r : 0;
@@ -82,7 +80,14 @@ bool to_sell(int32_t n, const RowLists &rl, HostSell *h) {
   }
   h->bandwidth = band;
   h->nnz = nnz;
-  h->far = far;
+  // a sample tells the share
+  const int32_t beyond = n / 16;
+  for (int32_t r = 0; r < n; r += 61)
+    for (int64_t k = rl.ptr[r]; k < rl.ptr[r + 1]; ++k) {
+      const int32_t c = rl.col[k];
+      h->far += (c > r ? c - r : r - c) > beyond;
+      ++h->far_of;
+    }
   return true;
 }
 
