@@ -1,13 +1,18 @@
-// Batched solves: many independent systems of uneven size in one persistent
-// cooperative launch, replayed from a CUDA graph.
+// Batched solves: many independent systems of uneven size in one graph launch.
 //
 // The systems are concatenated into one block-diagonal SELL-32 matrix, each
 // system's rows padded to whole slices so that no slice straddles two
-// systems.  Each system gets a team of blocks (persist.cuh): its own slice
-// range, reductions over its own blocks and its own bounded barrier, so every
-// system iterates at its own pace and stops at its own convergence inside the
-// single launch.  Blocks are shared out in proportion to each system's work
-// per solve (slices x iterations), which the autotuner measures.
+// systems.  Each system gets a team of blocks: its own slice range, sums over
+// its own blocks and its own bounded waits, so every system iterates at its own
+// pace and stops at its own convergence.
+//
+// PCG runs on the on-chip engine's teams (onchip.cu, mixed_team.cu) where they
+// hold the batch, in rounds: the kernel is the body of a graph's WHILE node,
+// and each round shares the blocks out anew over the systems left by a model of
+// a team's time (team_sync.cuh).  The rest, BiCGSTAB among it, is one persistent
+// cooperative launch with a barrier a team (persist.cuh), whose blocks are
+// shared out in proportion to each system's work per solve.  The autotuner
+// measures the work for both.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -578,8 +583,8 @@ int sfr_gpu_batch_create(int32_t nsys, const int32_t *neq, const int32_t *nad,
     }
     cat.bandwidth = std::max(cat.bandwidth, h.bandwidth);
     cat.max_width = std::max(cat.max_width, h.max_width);
-    cat.nnz += h.nnz;
     cat.far += h.far;
+    cat.far_of += h.far_of;
     rows += static_cast<int64_t>(h.nslices) * sfr::kWarpHost;
     slices += h.nslices;
     src += ns;
