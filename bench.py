@@ -64,10 +64,10 @@ def parse_args(argv=None):
                          "loop (profiling), 4 resident (mixed PCG)")
     ap.add_argument("--threads", type=int, default=0, help="graph-engine block size (0: default)")
     ap.add_argument("--spw", type=int, default=0, help="SELL slices per warp (0: default)")
-    ap.add_argument("--fused", type=int, default=4,
+    ap.add_argument("--fused", type=int, default=None,
                     help="graph engine FP64 PCG: 0 three kernels an iteration, 1-3 one "
-                         "cooperative kernel an iteration, 4 (the library's default) the whole "
-                         "solve in one cooperative launch")
+                         "cooperative kernel an iteration, 4 the whole solve in one cooperative "
+                         "launch (default: the library's own, the on-chip engine)")
     ap.add_argument("--pf", type=int, default=0,
                     help="graph engine SpMV-phase L2 prefetch distance in rounds (0: off)")
     ap.add_argument("--mixed", action="store_true", help="--profile solve: mixed precision")
@@ -228,7 +228,8 @@ def run_ours(args):
     g.set_engine(args.engine, args.threads, args.spw)
     if args.pf:
         g.set_prefetch(args.pf)
-    g.set_fused(args.fused)
+    if args.fused is not None:
+        g.set_fused(args.fused)
     stream = torch.cuda.Stream()
     sptr = stream.cuda_stream
     b = torch.tensor(s.b[0], device="cuda")
@@ -445,8 +446,10 @@ def run_ours(args):
 
     alg = pcg_alg_bytes(N, nnz, iters)
     achieved = alg / (ms_step * 1e-3) / 1e9
-    # the timed solves' engine: the autotuner's choice, or the flags given
-    fused = int(tune["headline_fp64"]["fused"]) if tune else int(args.fused)
+    # the timed solves' engine: the autotuner's choice, or the flags given, or
+    # the library's default (5 stands for the on-chip engine)
+    fused = (int(tune["headline_fp64"]["fused"]) if tune else
+             int(args.fused) if args.fused is not None else 5 if args.engine == 0 else 4)
     tr = committed_traffic("pcg_fp64_onchip_iteration" if fused == 5
                            else "pcg_fp64_fused_loop_iteration" if fused == 4
                            else "pcg_fp64_fused_iteration" if fused else "pcg_fp64_iteration")

@@ -59,7 +59,8 @@ extern "C" {
 /* FP32 matrix + inner Krylov, FP64 refinement.  BiCGSTAB on up to three
  * right-hand sides of a system that the on-chip engine holds runs there in
  * FP64 throughout, which is faster (refinements 0), unless an engine was
- * chosen (sfr_gpu_set_engine). */
+ * chosen (sfr_gpu_set_engine); where the true residual then misses the
+ * criterion, the mixed engine goes on with what is left of maxit. */
 #define SFR_MIXED 1
 
 typedef struct sfr_system sfr_system; /* one pattern resident on a device */
@@ -134,24 +135,36 @@ int sfr_gpu_solve_multi_device(sfr_system *s, int32_t solver, int32_t k, const d
                                int32_t newx, int32_t precision, void *stream,
                                sfr_solve_info *info);
 
-/* Choose how solves run: engine 0 = automatic (by size and solve), 1 = persistent
+/* Choose how solves run: engine 0 = automatic, 1 = persistent
  * (the whole solve in one cooperative launch: lowest latency, small
  * systems), 2 = graph (one full-occupancy kernel per phase inside a CUDA
  * graph whose iteration loop is a device-controlled conditional node: large
- * systems), 3 = the graph engine's kernels launched from a host loop for
+ * systems; FP64 PCG in the mode of sfr_gpu_set_fused), 3 = the graph engine's
+ * kernels launched from a host loop for
  * exactly maxit iterations (for profilers, which cannot look inside graphs
  * with conditional nodes; finished solves make the remaining launches
  * no-ops), 4 = resident (mixed-precision PCG with one right-hand side: one
  * cooperative launch with a block per SM, the symmetrically scaled FP32
- * operator with 16-bit column offsets held in L2 and the inner vectors in
- * shared memory; SFR_UNSUPPORTED for other solves, for a diagonal that is
- * not positive, a matrix bandwidth above 32767 or rows that do not fit the
- * blocks' shared memory -- about 2.8 million on a B200).  The automatic
- * choice takes the resident engine for mixed PCG from 100,000 rows when it
- * applies.  threads (128 or 256) and slices_per_warp (1..64; a SELL slice is
+ * operator with 16-bit column offsets held in L2 or shared memory and the inner
+ * vectors in shared memory; SFR_UNSUPPORTED for other solves, for a diagonal
+ * that is not positive, a matrix bandwidth above 32767 or rows that do not fit
+ * the blocks' shared memory -- about 2.8 million on a B200).
+ *
+ * The automatic choice, in this order: the resident engine for mixed PCG with
+ * one right-hand side from 512 rows when it applies; the on-chip engine for
+ * FP64 PCG with one right-hand side where the system fits it and
+ * sfr_gpu_set_fused was never called; the on-chip engine for BiCGSTAB, FP64 or
+ * mixed, with up to three right-hand sides where the system fits it; else the
+ * persistent engine below 100,000 rows and the graph engine above.  No engine
+ * number stands for the on-chip engine.
+ *
+ * threads (128 or 256) and slices_per_warp (1..64; a SELL slice is
  * 32 rows) set the graph engine's launch shape; 0 keeps the current value;
  * slices_per_warp = -1 (the default) sizes the SpMV phases to one wave of
- * the blocks resident on the GPU at once. */
+ * the blocks resident on the GPU at once.  They, sfr_gpu_set_prefetch and
+ * sfr_gpu_set_staging reach the solves that run on the graph engine's kernels,
+ * which under engine 0 are those the last rule leaves it.  Transposed solves
+ * and adjoints run with the same settings. */
 int sfr_gpu_set_engine(sfr_system *s, int32_t engine, int32_t threads,
                        int32_t slices_per_warp);
 
@@ -171,15 +184,19 @@ int sfr_gpu_set_prefetch(sfr_system *s, int32_t rounds);
  * broadcasts the total in one epoch-tagged word that the others poll; mode
  * 4 runs mode 3's iteration in a loop inside one cooperative launch for the
  * whole solve, each block waiting after its update of p only on the blocks
- * whose p its next SpMV phase gathers.  Solves it
- * does not serve (other solvers, K > 1, mixed precision, or no co-resident
- * shape) take the three-kernel iteration; 0 turns the fused iteration off
- * (three kernels an iteration); other values are SFR_BAD_INPUT.  Under
- * the automatic choice (engine 0), a handle this was never called for solves
- * FP64 PCG with one right-hand side on the on-chip engine (one launch a solve, one reduction an iteration, the Krylov
- * vectors in shared memory; small systems wholly inside one thread-block
- * cluster), or in mode 4 where the system does not fit it; sfr_tune_result
- * reports it as mode 5.  Under engine 2 mode 4 is the default. */
+ * whose p its next SpMV phase gathers.  Solves it does not serve (other
+ * solvers, K > 1, mixed precision, or no co-resident shape) take the
+ * three-kernel iteration; 0 turns the fused iteration off (three kernels an
+ * iteration); other values are SFR_BAD_INPUT.  Under engine 2 mode 4 is the
+ * default.
+ *
+ * Under the automatic choice a handle this was never called for solves FP64
+ * PCG with one right-hand side on the on-chip engine (one launch a solve, one
+ * reduction an iteration, the Krylov vectors in shared memory; small systems
+ * wholly inside one thread-block cluster), or in mode 4 where the system does
+ * not fit it; sfr_tune_result reports it as mode 5.  A call takes the handle's
+ * PCG off the on-chip engine for good (a tuned choice of it aside); BiCGSTAB
+ * is not concerned. */
 int sfr_gpu_set_fused(sfr_system *s, int32_t mode);
 
 /* Graph engine, BiCGSTAB: 1 stages each warp's SELL slices (slot values and
@@ -194,11 +211,12 @@ int sfr_gpu_set_staging(sfr_system *s, int32_t flag);
 
 /* Result of sfr_gpu_autotune. */
 typedef struct {
-  int32_t engine;           /* chosen engine: 1 persistent, 2 graph, 4 resident */
+  int32_t engine;           /* chosen engine: 1 persistent, 2 graph, 4 resident; the on-chip
+                               engine is 2 with fused 5, for mixed BiCGSTAB 0 with fused 5 */
   int32_t threads;          /* graph engine block size */
   int32_t slices_per_warp;  /* graph engine SpMV phases: 0 one wave, else slices per warp */
   int32_t prefetch;         /* graph engine SpMV-phase L2 prefetch distance (rounds) */
-  int32_t fused;            /* graph engine FP64 PCG: one kernel an iteration (mode) */
+  int32_t fused;            /* sfr_gpu_set_fused's mode; 5: the on-chip engine */
   double ms;                /* the choice's solve time (ms, CUDA events) */
   int32_t default_engine, default_threads, default_slices_per_warp, default_prefetch,
       default_fused;
@@ -270,9 +288,11 @@ typedef struct sfr_batch sfr_batch; /* many systems solved in one launch */
 
 /* Upload nsys patterns of one storage kind (arrays of per-system pointers,
  * each system as sfr_gpu_create takes it).  The systems are concatenated
- * block-diagonally; one persistent cooperative launch (replayed from a CUDA
- * graph) solves them all, each system by its own team of thread blocks with
- * its own barrier, so each stops at its own convergence.  No counterpart in
+ * block-diagonally and solved together, each by its own team of thread blocks
+ * with its own exchanges, so each stops at its own convergence: PCG on the
+ * on-chip engine's teams where they fit, in rounds of a CUDA graph's loop that
+ * share the blocks out anew over the systems left; else one persistent
+ * cooperative launch (replayed from a CUDA graph).  No counterpart in
  * the reference, which solves systems one solverC call at a time. */
 int sfr_gpu_batch_create(int32_t nsys, const int32_t *neq, const int32_t *nad,
                          const int32_t *const *ia, const int32_t *const *ja,

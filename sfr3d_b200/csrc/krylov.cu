@@ -896,7 +896,7 @@ int auto_engine(sfr_system *s, int32_t solver, int32_t k, int32_t precision, boo
   const bool resident_case = precision == SFR_MIXED && solver == SFR_PCG && k == 1 && own_diag;
   if (resident_case && s->n >= kResidentRows && resident_fits(s)) return 4;
   if (precision == SFR_FP64 && solver == SFR_PCG && k == 1 && s->graph_fused == kFusedOnChip)
-    return 2;  // the on-chip engine, at every size
+    return 2;  // the on-chip engine (mode 4 past what it holds)
   if (onchip_bicg_case(solver, precision, 0, nullptr) && onchip_bicg_fits(s, k, own_diag))
     return precision == SFR_FP64 ? 2 : 0;
   return s->n >= kGraphEngineRows ? 2 : 1;

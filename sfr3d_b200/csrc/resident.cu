@@ -6,8 +6,8 @@
 // couplings and 16-bit column offsets, is 75 MB and stays in L2 from one
 // iteration to the next; the FP64 operator (150 MB) cannot.  One cooperative
 // launch runs the whole solve with one block per SM (fewer below 16 slices a
-// block).  A system whose operator fits shared memory too (up to about 64^3)
-// keeps it there, and an iteration then reads only p from L2: with the
+// block).  A system whose operator fits shared memory too (six neighbours a
+// row: up to about 86^3) keeps it there, and an iteration then reads only p from L2: with the
 // exchange of team_sync.cuh an iteration went from 6.6 to 4.4 us at 24^3, from
 // 6.9 to 5.9 at 48^3, from 8.0 to 7.3 at 64^3, from 13.2 to 12.8 at 96^3 and
 // from 24.8 to 24.0 at 128^3.  Each block owns a

@@ -249,8 +249,9 @@ class GpuSystem:
         """Graph engine, FP64 PCG with one right-hand side
         (sfr_gpu_set_fused): 0 three kernels an iteration, 1-3 one cooperative
         kernel an iteration (2: held to 40 registers; 3: tagged exchanges),
-        4 the whole solve in one cooperative launch.  A system this was never
-        called for takes the on-chip engine, mode 4 where it does not fit."""
+        4 the whole solve in one cooperative launch.  Under the automatic
+        choice a system this was never called for takes the on-chip engine,
+        mode 4 where it does not fit; under engine 2 mode 4 is the default."""
         rc = lib().sfr_gpu_set_fused(self.h, int(mode))
         if rc != OK:
             raise SolverError(rc, "sfr_gpu_set_fused")
