@@ -78,6 +78,8 @@ struct PinnedPool {
       if (cudaHostAlloc(&p, sizeof(SolveOut) * kRecords,
                         cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess)
         base = static_cast<SolveOut *>(p);
+      else
+        (void)cudaGetLastError();  // the refusal is not a later call's error
     }
     if (!base || used == ~0ull) return nullptr;
     const int i = __builtin_ctzll(~used);
