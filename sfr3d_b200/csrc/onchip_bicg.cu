@@ -480,8 +480,11 @@ size_t live_line(const sfr_system *s, int k, size_t op, size_t live) {
 // iteration with 190 KB at most and with all of it: 52^3 of 3 37 and 54, 60^3 of
 // 3 50 and 78, 64^3 of 2 42 and 66, 84^3 of 1 47 and 74, 88^3 of 1 53 and 84
 // (the streaming engine: 72, 88, 71, 74 and 80).  Numbered, the vectors that
-// leave cost more than the L1 gives: 76^3 of 3 63 with all, 75 without.
-constexpr size_t kFarSmem = (196 << 10) - 1024;
+// leave cost more than the L1 gives: 76^3 of 3 63 with all, 75 without.  So does
+// the operator of a system whose z is about as small as that L1 (kFarZ): random
+// rows of 20, 2,000 of 2 (32 KB) 23.4 with all, 27.2 without, 4,000 of 2 (64 KB)
+// 32.0 and 21.6, 6,000 of 1 (48 KB) 21.1 and 19.4.
+constexpr size_t kFarSmem = (196 << 10) - 1024, kFarZ = 40 << 10;
 
 template <typename I, int K>
 bool shape_of(const sfr_system *s, bool own_diag, Shape *sh) {
@@ -490,7 +493,8 @@ bool shape_of(const sfr_system *s, bool own_diag, Shape *sh) {
       cudaSuccess)
     return false;
   const size_t most = static_cast<size_t>(optin) - kStatic;
-  const size_t limit = s->A.far() ? std::min(most, kFarSmem - kStatic) : most;
+  const bool far = s->A.far() && sizeof(double) * K * static_cast<size_t>(s->n) > kFarZ;
+  const size_t limit = far ? std::min(most, kFarSmem - kStatic) : most;
   const int ns = s->A.nslices;
   const int g = std::max(1, std::min(num_sms(s->device), (ns + kBlockSlices - 1) / kBlockSlices));
   const int slices = (ns + g - 1) / g;
