@@ -114,8 +114,8 @@ std::vector<int> share_by_weight(const sfr_batch *b, int gmax) {
 // 52, 54 and 88, 58, 54, 52 (the persistent kernels: 112 and 128, 28.1 and 28.6,
 // 82 and 96).
 constexpr int kFarSmem = 164 << 10;
-// ... and mixed teams that hold their vectors in it (plan).
-constexpr int kMixedSmem = 196 << 10;
+// ... and the carve-out above, for teams that hold enough in it (plan).
+constexpr int kHoldSmem = 196 << 10;
 
 // A block's dynamic shared memory where the SM's is `sm` bytes: less the team
 // kernels' static shared memory and the 1 KB the system takes of each block.
@@ -135,6 +135,12 @@ std::vector<int> least_blocks(const sfr_batch *b, const TeamShape &sh) {
   if (sh.most > 0)
     for (int s = 0; s < b->nsys; ++s) nb[s] = std::max(1, (b->nslices[s] + sh.most - 1) / sh.most);
   return nb;
+}
+
+// Shared memory of a slice with all of its rows' vectors and its slots.
+int64_t slice_bytes(const sfr_batch *b, int row, int value) {
+  const int64_t slots = b->cat.A.max_width;
+  return kWarpHost * (row + slots * (value + (b->cat.A.off ? 2 : 4))) + 4;
 }
 
 // Slices of which a block of the mixed teams' has room for `vecs` FP32 vectors
@@ -296,19 +302,28 @@ int plan(sfr_batch *b, int32_t solver, int32_t precision) {
   // -> 39.4 ms (the persistent kernels 37.9), of 80^3 16.8 -> 14.8, 8 of 48^3 9.3
   // -> 8.3.  Teams that lose more lose time: r, 2 boxes of 128^3 144 -> 158; the
   // operator, 148 of 12^3 0.80 -> 1.02, 16 of 32^3 4.5 -> 5.0.
+  int widest = 0;  // slices of a block
+  for (int s = 0; s < S; ++s) widest = std::max(widest, (b->nslices[s] + nb[s] - 1) / nb[s]);
   if (e == kChipMixed) {
     TeamShape small = shape;
-    small.smem = std::min(shape.smem, team_smem(kMixedSmem, shape.per_sm));
+    small.smem = std::min(shape.smem, team_smem(kHoldSmem, shape.per_sm));
     small.most = mixed_slices(small, 1);
-    // all of a slice: its rows' vectors and its slots
-    const int whole = kWarpHost * (24 + b->cat.A.max_width * (b->cat.A.off ? 6 : 8)) + 4;
-    const auto room = [&](const TeamShape &sh) { return static_cast<int>(sh.smem - 32) / whole; };
-    bool same = true;
+    const int64_t whole = slice_bytes(b, 24, 4);
+    bool same = widest <= mixed_slices(small, 3);
     for (int s = 0; s < S; ++s) {
-      const int w = (b->nslices[s] + nb[s] - 1) / nb[s];
-      same = same && w <= mixed_slices(small, 3) && (w <= room(small) || w > room(shape));
+      const int64_t need = (b->nslices[s] + nb[s] - 1) / nb[s] * whole + 32;
+      same = same && (need <= static_cast<int64_t>(small.smem) ||
+                      need > static_cast<int64_t>(shape.smem));
     }
     if (same) shape = small;
+  }
+  // Unnumbered FP64 teams that hold their operators in the 196 KB carve-out and
+  // not in 164: 64 boxes of 12^3 0.51 ms, 0.58 without.
+  if (e == kChipFp64 && b->cat.A.far()) {
+    const int64_t need = widest * slice_bytes(b, 40, 8) + 32;
+    const size_t hold = team_smem(kHoldSmem, shape.per_sm);
+    if (need > static_cast<int64_t>(shape.smem) && need <= static_cast<int64_t>(hold))
+      shape.smem = hold;
   }
   std::vector<int4> blocks;
   std::vector<int2> sys;
