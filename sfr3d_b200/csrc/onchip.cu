@@ -16,7 +16,8 @@
 // none.  p then keeps a few eps of the old direction beside a z many orders
 // larger than that, and the solve goes on as the reference's (a right-hand side
 // of one eigenvector and 1e-11 of noise: the same count of iterations).  An
-// iteration is then SpMV, exchange, update, publication of p: two synchronisations instead of three, and no vector but p leaves the chip.
+// iteration is then SpMV, exchange, update, publication of p: two
+// synchronisations instead of three, and no vector but p leaves the chip.
 // Every SpMV row keeps the reference's rounding and order (diagonal product,
 // then each slot).  A solve runs one SpMV phase beyond its last update, the
 // one that measures the residual it stops on.

@@ -7,16 +7,16 @@
 // iteration to the next; the FP64 operator (150 MB) cannot.  One cooperative
 // launch runs the whole solve with one block per SM (fewer below 16 slices a
 // block).  A system whose operator fits shared memory too (six neighbours a
-// row: up to about 86^3) keeps it there, and an iteration then reads only p from L2: with the
-// exchange of team_sync.cuh an iteration went from 6.6 to 4.4 us at 24^3, from
-// 6.9 to 5.9 at 48^3, from 8.0 to 7.3 at 64^3, from 13.2 to 12.8 at 96^3 and
-// from 24.8 to 24.0 at 128^3.  Each block owns a
-// contiguous range of SELL slices and keeps, for its rows, the inner
-// residual, the FP32 solution increment, A p and (when it fits) the
-// diagonal correction in shared memory (16 bytes a row).  The global traffic
-// of an inner iteration is the operator (from L2), the gathers of p and the
-// update of p; one exchange of partial sums separates its two phases, and a
-// wait on the blocks whose p the next SpMV phase gathers ends it.
+// row: up to about 86^3) keeps it there, and an iteration then reads only p
+// from L2: with the exchange of team_sync.cuh an iteration went from 6.6 to 4.4
+// us at 24^3, from 6.9 to 5.9 at 48^3, from 8.0 to 7.3 at 64^3, from 13.2 to
+// 12.8 at 96^3 and from 24.8 to 24.0 at 128^3.  Each block owns a contiguous
+// range of SELL slices and keeps, for its rows, the inner residual, the FP32
+// solution increment, A p and (when it fits) the diagonal correction in shared
+// memory (16 bytes a row).  The global traffic of an inner iteration is the
+// operator (from L2), the gathers of p and the update of p; one exchange of
+// partial sums separates its two phases, and a wait on the blocks whose p the
+// next SpMV phase gathers ends it.
 //
 // Arithmetic.  PCG with the Jacobi preconditioner M = diag(1/ad) (Cg.c:47-209,
 // PreCond.c:18-26) is CG on the symmetrically scaled system
